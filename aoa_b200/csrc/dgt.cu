@@ -102,7 +102,7 @@ __global__ void gi_twist(uint64_t* data, long poly_stride, int npolys, int first
   const uint64_t q = pc[prime].q;
   const uint64_t* w = tab + (long)prime * 6 * H + n;
   const uint64_t a = x[n], b = x[H + n];
-  if (q < (1ull << kLazyPrimeBits)) {      // the prime is the same for the whole block
+  if (lazy_prime(q)) {                     // the prime is the same for the whole block
     if ((q & 0xffffffffull) == 1) gi_twist_lazy<true>(x, n, H, w, a, b, q, lazy_out);
     else gi_twist_lazy<false>(x, n, H, w, a, b, q, lazy_out);
     return;

@@ -284,7 +284,7 @@ int aoa_engine_create(const aoa_params* p, aoa_engine** out) {
         if (E.primes[i] == E.primes[j]) throw AoaError(AOA_ERR_BAD_PARAM, "primes must be distinct");
     E.prime_kind.clear();
     for (uint64_t q : E.primes) {
-      const int kind = q >= (1ull << kLazyPrimeBits) ? kButterflyCanonical
+      const int kind = !lazy_prime(q) ? kButterflyCanonical
                        : (q & 0xffffffffull) == 1 ? kButterflyLazyQ1 : kButterflyLazy;
       E.prime_kind.push_back((char)kind);
     }

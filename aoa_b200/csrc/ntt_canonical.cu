@@ -1,0 +1,6 @@
+// The pass kernels of one butterfly kind (ntt_kernels.cuh).
+#include "ntt_kernels.cuh"
+
+namespace aoa {
+AOA_NTT_KIND(, kButterflyCanonical)
+}  // namespace aoa
