@@ -46,6 +46,9 @@ constexpr int kLazyPrimeBits = AOA_LAZY_PRIME_BITS;
 constexpr uint64_t kLazyPrimeMin = 1ull << 34;
 __host__ __device__ inline bool lazy_prime(uint64_t q) { return q >= kLazyPrimeMin && q < (1ull << kLazyPrimeBits); }
 constexpr int kButterflyCanonical = 0, kButterflyLazy = 1, kButterflyLazyQ1 = 2;
+// Output primes from here up take one 32-bit Montgomery step in the tensor-core
+// conversion's epilogue (its result is below q + 2^49)
+constexpr uint64_t kConvMontgomeryMin = 1ull << 50;
 constexpr int kLargeItems = 1536;           // limb-transform launches this large use ntt_waves_large
 
 struct Tune {

@@ -180,13 +180,14 @@ static void build_rns_tables(Engine& E) {
     for (int i = 0; i < l; i++) resc[(size_t)l * k + i] = sh(h_invmod(P[l] % P[i], P[i]), P[i]);
   if (k <= 32 && kl >= 1 && kl <= 32 && E.N % 128 == 0) {
     // [16 k-chunks][256 columns][16 B]: byte k = 8 in + a of column n = 8 out + b
-    // holds byte b of h 2^(8a) mod p_out (the conversion kernel's B operand)
+    // holds byte b of h 2^(8a) mod p_out, times 2^32 where the epilogue reduces
+    // by a Montgomery step (the conversion kernel's B operand)
     constexpr size_t kImg = 65536;
     auto image = [](const uint64_t* mat, int ld, int nin, int nout, const uint64_t* outp, uint8_t* img) {
       for (int out = 0; out < nout; out++) {
         const uint64_t p = outp[out];
         uint64_t sh[8];
-        sh[0] = 1 % p;
+        sh[0] = p >= kConvMontgomeryMin ? (1ull << 32) % p : 1 % p;   // cancels the epilogue's Montgomery step
         for (int a = 1; a < 8; a++) sh[a] = h_mulmod(sh[a - 1], 256 % p, p);
         for (int in = 0; in < nin; in++) {
           const uint64_t h = mat[(size_t)in * ld + out] % p;

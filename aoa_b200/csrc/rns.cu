@@ -202,18 +202,24 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// sum_b T_b 2^(8b) (b < 8, T_b < 2^24) reduced mod P.  W_0 = sum_t T_t 2^(8t)
-// and W_1 = sum_t T_(4+t) 2^(8t) (< 2^49 each) come from 32 x 32 -> 64-bit
-// multiply-adds; x = W_0 + W_1 2^32 < 2^81 has a high word below 2^17, so
-// one Barrett step (s >= 32) reduces it.
-// an output prime's constants, staged in shared memory once per CTA
+// an output prime's constants, staged in shared memory once per CTA; minv =
+// -q^-1 mod 2^32 for primes reduced by a Montgomery step, else 0
 struct TcOut {
-  uint64_t q, mu, sh, one_sh;
+  uint64_t q, mu, one_sh;
+  uint32_t sh, minv;
 };
 
-// Q1: every input and output prime of the launch is q = 1 mod 2^32 below
-// 2^60 (the engine's butterfly kind kButterflyLazyQ1): the quotient times q
-// in the reductions and Shoup products takes one 32-bit multiply (mul_q1).
+// sum_b T_b 2^(8b) (b < 8, T_b < 2^24) reduced mod P.  W_0 = sum_t T_t 2^(8t)
+// and W_1 = sum_t T_(4+t) 2^(8t) (< 2^49 each) come from 32 x 32 -> 64-bit
+// multiply-adds; x = W_0 + W_1 2^32 < 2^81.  For q >= kConvMontgomeryMin the
+// table holds 2^32 times its entries and one Montgomery step takes the factor
+// back: with m = -W_0 q^-1 mod 2^32, (x + m q) / 2^32 = W_1 + ceil part < q +
+// 2^49, one conditional subtraction from [0, q).  For q = 1 mod 2^32 (Q1: every
+// input and output prime of the launch, kButterflyLazyQ1) m is -W_0 mod 2^32
+// and x - w q with w = W_0 mod 2^32 takes a single wide multiply.  Smaller
+// primes take one Barrett step (s >= 32) or the general reduction.  The kernel
+// is bound by this CUDA-core work: against a Barrett step for every prime (a
+// 64-bit high product and two subtractions), 48 HMults at 2^16 10574 -> 10327 us.
 template <bool Q1>
 __device__ __forceinline__ uint64_t tc_combine(const uint32_t* v, const TcOut& c, const PrimeConst* P) {
   uint64_t W0 = v[0], W1 = v[4];
@@ -223,13 +229,24 @@ __device__ __forceinline__ uint64_t tc_combine(const uint32_t* v, const TcOut& c
   asm("mad.wide.u32 %0, %1, 65536, %0;" : "+l"(W1) : "r"(v[6]));
   asm("mad.wide.u32 %0, %1, 16777216, %0;" : "+l"(W0) : "r"(v[3]));
   asm("mad.wide.u32 %0, %1, 16777216, %0;" : "+l"(W1) : "r"(v[7]));
+  if (c.minv) {
+    uint64_t r;
+    if (Q1) {
+      r = W1 + (W0 >> 32) + c.q - (uint64_t)(uint32_t)W0 * (uint32_t)(c.q >> 32);
+    } else {
+      const uint32_t m = (uint32_t)W0 * c.minv;
+      const uint64_t a = (uint64_t)m * (uint32_t)c.q + (uint32_t)W0;                    // low word 0
+      r = W1 + (W0 >> 32) + (uint64_t)m * (uint32_t)(c.q >> 32) + (a >> 32);
+    }
+    return r >= c.q ? r - c.q : r;
+  }
   uint32_t r1, r2;
   asm("add.cc.u32 %0, %2, %3;\n\t"
       "addc.u32 %1, %4, 0;"
       : "=r"(r1), "=r"(r2)
       : "r"((uint32_t)(W0 >> 32)), "r"((uint32_t)W1), "r"((uint32_t)(W1 >> 32)));
   const uint64_t lo = ((uint64_t)r1 << 32) | (uint32_t)W0;
-  if (c.sh) return Q1 ? barrett_wide_q1(lo, r2, c.q, c.mu, (uint32_t)c.sh) : barrett_wide(lo, r2, c.q, c.mu, (uint32_t)c.sh);
+  if (c.sh) return Q1 ? barrett_wide_q1(lo, r2, c.q, c.mu, c.sh) : barrett_wide(lo, r2, c.q, c.mu, c.sh);
   return reduce128(lo, r2, *P);
 }
 
@@ -249,6 +266,11 @@ __device__ __forceinline__ uint64_t tc_scale(uint64_t x, ShoupW w, uint64_t q) {
     r = r >= 2 * q ? r - 2 * q : r;
     return r >= q ? r - q : r;
   } else {
+    if (q < (1ull << kLazyPrimeBits)) {
+      uint64_t r = shoup_lazy_mad3(x, w.w, w.wp, 0 - q);
+      r = r >= 2 * q ? r - 2 * q : r;
+      return r >= q ? r - q : r;
+    }
     return shoup(x, w, q);
   }
 }
@@ -298,7 +320,8 @@ basis_convert_tc(ConvArgs a, int j_first, int j_end) {
     }
     if (i < j_end) {
       const PrimeConst& P = a.pc[a.out_prime0 + i];
-      s_out[i] = TcOut{P.q, P.bar_mu, P.bar_sh, P.one_sh};
+      s_out[i] = TcOut{P.q, P.bar_mu, P.one_sh, (uint32_t)P.bar_sh,
+                       P.q >= kConvMontgomeryMin ? (uint32_t)P.qinv_neg : 0};
     }
   }
   if (warp == 0) {
