@@ -68,4 +68,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mb, unsigned parity, int lim
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// In a kernel launched with launch_pdl, before anything but constants is read
+// or anything is written: waits for the stream's previous kernel to complete
+// (its writes are visible afterwards), then lets the next one be set up.  In
+// this order at most one kernel waits on the SMs ahead of its turn.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 }  // namespace aoa

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "aoa_internal.h"
+#include "async.cuh"
 
 using namespace aoa;
 
@@ -94,6 +95,7 @@ __device__ __forceinline__ void gi_twist_lazy(uint64_t* x, int n, int H, const u
 
 __global__ void gi_twist(uint64_t* data, long poly_stride, int npolys, int first_prime, const uint64_t* __restrict__ tab,
                          int H, const PrimeConst* __restrict__ pc, bool lazy_out) {
+  pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   const int item = blockIdx.y, limb = item / npolys, p = item % npolys;
@@ -127,6 +129,7 @@ __device__ __forceinline__ void gi_mul_dev(uint64_t ar, uint64_t ai, uint64_t br
 // c = a * b element-wise on GI limbs (mul_dgt<GaussianInteger>, dgt.cu:1327-1341).
 __global__ void gi_mul(uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* b, long bs, int prime0,
                        int npolys, int H, const PrimeConst* __restrict__ pc) {
+  pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   const int item = blockIdx.y, limb = item / npolys, p = item % npolys;
@@ -164,6 +167,7 @@ __device__ __forceinline__ void gi_tensor_at(const uint64_t* a, long a_half, con
 
 __global__ void gi_tensor(const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0, uint64_t* d1,
                           uint64_t* d2, int H, const PrimeConst* __restrict__ pc) {
+  pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   gi_tensor_at(a, a_half, b, b_half, d0, d1, d2, H, pc, n, blockIdx.y);
@@ -173,6 +177,7 @@ __global__ void gi_tensor(const uint64_t* a, long a_half, const uint64_t* b, lon
 // ([c0 | c1], stride half), outputs D0 = D, D1 = D + n half, D2 = D + 2n half
 // at op stride half
 __global__ void gi_tensor_batch(CtPtrs ptr, long half, uint64_t* D, int nops, int H, const PrimeConst* __restrict__ pc) {
+  pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   const int z = blockIdx.z;
@@ -203,6 +208,7 @@ __device__ __forceinline__ void gi_keyswitch_at(const uint64_t* xq, const uint64
 
 __global__ void gi_keyswitch_mul(const uint64_t* xq, const uint64_t* xb, const uint64_t* key, long key_half,
                                  uint64_t* k0, uint64_t* k1, int nq, int K, int H, const PrimeConst* __restrict__ pc) {
+  pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   gi_keyswitch_at(xq, xb, key, key_half, k0, k1, nq, K, H, pc, n, blockIdx.y);
@@ -213,6 +219,7 @@ __global__ void gi_keyswitch_mul(const uint64_t* xq, const uint64_t* xb, const u
 __global__ void gi_keyswitch_mul_batch(const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
                                        const uint64_t* key, long key_half, uint64_t* k, long k_stride, int nops,
                                        int nq, int K, int H, const PrimeConst* __restrict__ pc) {
+  pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   const int z = blockIdx.z;
@@ -222,6 +229,7 @@ __global__ void gi_keyswitch_mul_batch(const uint64_t* xq, long xq_stride, const
 
 // Reference GaussianInteger layout <-> planar GI limbs.
 __global__ void gi_layout(uint64_t* dst, const uint64_t* src, int H, bool to_planar) {
+  pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   const long base = (long)blockIdx.y * 2 * H;
@@ -352,16 +360,14 @@ void dgt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int
   if (forward) {
     // the limb transforms of rings of 2^11 and more take forward inputs below
     // 16q on their lazy limbs (the smaller ones run canonical butterflies)
-    gi_twist<<<gi_grid(E, nlimbs * npolys), 256, 0, st>>>(data, poly_stride * E.N, npolys, first_prime, E.d_twist,
+    launch_pdl(gi_twist, gi_grid(E, nlimbs * npolys), 256, 0, st, data, poly_stride * E.N, npolys, first_prime, E.d_twist,
                                                             H, E.d_pc, T.log_n >= 10);
-    note_launch();
     AOA_CHECK_LAUNCH();
     ntt_batch_tables(E, T, data, npolys, first_prime, 2 * nlimbs, 2 * poly_stride, true, st);
   } else {
     ntt_batch_tables(E, T, data, npolys, first_prime, 2 * nlimbs, 2 * poly_stride, false, st);
-    gi_twist<<<gi_grid(E, nlimbs * npolys), 256, 0, st>>>(data, poly_stride * E.N, npolys, first_prime,
+    launch_pdl(gi_twist, gi_grid(E, nlimbs * npolys), 256, 0, st, data, poly_stride * E.N, npolys, first_prime,
                                                             E.d_untwist, H, E.d_pc, false);
-    note_launch();
     AOA_CHECK_LAUNCH();
   }
 }
@@ -369,23 +375,20 @@ void dgt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int
 void gi_mul_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* b, long bs,
                int prime0, int nlimbs, int npolys, cudaStream_t st) {
   if (nlimbs <= 0 || npolys <= 0) return;
-  gi_mul<<<gi_grid(E, nlimbs * npolys), 256, 0, st>>>(c, cs, a, as, b, bs, prime0, npolys, (int)(E.N / 2), E.d_pc);
-  note_launch();
+  launch_pdl(gi_mul, gi_grid(E, nlimbs * npolys), 256, 0, st, c, cs, a, as, b, bs, prime0, npolys, (int)(E.N / 2), E.d_pc);
   AOA_CHECK_LAUNCH();
 }
 
 void gi_tensor_op(const Engine& E, const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0,
                   uint64_t* d1, uint64_t* d2, int nlimbs, cudaStream_t st) {
-  gi_tensor<<<gi_grid(E, nlimbs), 256, 0, st>>>(a, a_half, b, b_half, d0, d1, d2, (int)(E.N / 2), E.d_pc);
-  note_launch();
+  launch_pdl(gi_tensor, gi_grid(E, nlimbs), 256, 0, st, a, a_half, b, b_half, d0, d1, d2, (int)(E.N / 2), E.d_pc);
   AOA_CHECK_LAUNCH();
 }
 
 void gi_tensor_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D, int n, int nlimbs,
                         cudaStream_t st) {
   const dim3 g = gi_grid(E, nlimbs);
-  gi_tensor_batch<<<dim3(g.x, g.y, n), 256, 0, st>>>(ptr, half, D, n, (int)(E.N / 2), E.d_pc);
-  note_launch();
+  launch_pdl(gi_tensor_batch, dim3(g.x, g.y, n), 256, 0, st, ptr, half, D, n, (int)(E.N / 2), E.d_pc);
   AOA_CHECK_LAUNCH();
 }
 
@@ -393,18 +396,16 @@ void gi_keyswitch_mul_batch_op(const Engine& E, const uint64_t* xq, long xq_stri
                                long xb_stride, const uint64_t* key, uint64_t* k, long k_stride, int n, int nq,
                                cudaStream_t st) {
   const dim3 g = gi_grid(E, nq + E.kl);
-  gi_keyswitch_mul_batch<<<dim3(g.x, g.y, n), 256, 0, st>>>(xq, xq_stride, xb, xb_stride, key,
+  launch_pdl(gi_keyswitch_mul_batch, dim3(g.x, g.y, n), 256, 0, st, xq, xq_stride, xb, xb_stride, key,
                                                               (long)(E.k + E.kl) * E.N, k, k_stride, n, nq, E.k,
                                                               (int)(E.N / 2), E.d_pc);
-  note_launch();
   AOA_CHECK_LAUNCH();
 }
 
 void gi_keyswitch_mul_op(const Engine& E, const uint64_t* xq, const uint64_t* xb, const uint64_t* key, uint64_t* k0,
                          uint64_t* k1, int nq, cudaStream_t st) {
-  gi_keyswitch_mul<<<gi_grid(E, nq + E.kl), 256, 0, st>>>(xq, xb, key, (long)(E.k + E.kl) * E.N, k0, k1, nq, E.k,
+  launch_pdl(gi_keyswitch_mul, gi_grid(E, nq + E.kl), 256, 0, st, xq, xb, key, (long)(E.k + E.kl) * E.N, k0, k1, nq, E.k,
                                                           (int)(E.N / 2), E.d_pc);
-  note_launch();
   AOA_CHECK_LAUNCH();
 }
 
@@ -449,8 +450,7 @@ int aoa_gi_to_planar(aoa_ctx* c, uint64_t* d_dst, const uint64_t* d_src, int nli
   return guarded([&] {
     const Engine& E = *c->c.E;
     if (nlimbs <= 0) return;
-    gi_layout<<<gi_grid(E, nlimbs), 256, 0, c->c.stream>>>(d_dst, d_src, (int)(E.N / 2), true);
-    note_launch();
+    launch_pdl(gi_layout, gi_grid(E, nlimbs), 256, 0, c->c.stream, d_dst, d_src, (int)(E.N / 2), true);
     AOA_CHECK_LAUNCH();
   });
 }
@@ -460,8 +460,7 @@ int aoa_gi_from_planar(aoa_ctx* c, uint64_t* d_dst, const uint64_t* d_src, int n
   return guarded([&] {
     const Engine& E = *c->c.E;
     if (nlimbs <= 0) return;
-    gi_layout<<<gi_grid(E, nlimbs), 256, 0, c->c.stream>>>(d_dst, d_src, (int)(E.N / 2), false);
-    note_launch();
+    launch_pdl(gi_layout, gi_grid(E, nlimbs), 256, 0, c->c.stream, d_dst, d_src, (int)(E.N / 2), false);
     AOA_CHECK_LAUNCH();
   });
 }

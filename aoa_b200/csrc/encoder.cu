@@ -22,6 +22,7 @@
 // enters as inputs (signed u, e1, e2 per coefficient), so results are
 // deterministic and comparable with the reference given the same draws.
 #include "aoa_internal.h"
+#include "async.cuh"
 
 using namespace aoa;
 
@@ -78,6 +79,7 @@ __device__ __forceinline__ void fwd_bf(double2& x, double2& y, unsigned j, unsig
 template <bool INV>
 __global__ void fft_stage(double2* v, unsigned size, unsigned len, const double2* __restrict__ ksi,
                           const uint32_t* __restrict__ rot, unsigned M) {
+  pdl_begin();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= size / 2) return;
   const unsigned lenh = len >> 1;
@@ -93,6 +95,7 @@ __global__ void fft_stage(double2* v, unsigned size, unsigned len, const double2
 // Inverse stages len = tile .. 2 on one tile of `tile` consecutive entries.
 __global__ void fft_inv_tile(double2* v, unsigned tile, const double2* __restrict__ ksi,
                              const uint32_t* __restrict__ rot, unsigned M) {
+  pdl_begin();
   extern __shared__ double2 sv[];
   double2* g = v + (size_t)blockIdx.x * tile;
   for (unsigned i = threadIdx.x; i < tile; i += blockDim.x) sv[i] = g[i];
@@ -120,6 +123,7 @@ __global__ void fft_fwd_tile_from_message(double2* v, const uint64_t* __restrict
                                           int log_size, unsigned tile, unsigned gap, unsigned half_n,
                                           const double2* __restrict__ ksi, const uint32_t* __restrict__ rot,
                                           unsigned M) {
+  pdl_begin();
   extern __shared__ double2 sv[];
   const unsigned base = blockIdx.x * tile;
   for (unsigned i = threadIdx.x; i < tile; i += blockDim.x) {
@@ -151,6 +155,7 @@ __device__ __forceinline__ uint64_t adjust_neg(int64_t x, const PrimeConst& P) {
 // positions), from the inverse-FFT output in bit-reversed order.
 __global__ void encode_residues(uint64_t* out, const double2* __restrict__ v, const PrimeConst* __restrict__ pc,
                                 unsigned N, int log_size, unsigned gap, double size_d, double scale_d) {
+  pdl_begin();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   const int lid = blockIdx.y;
   if (t >= N) return;
@@ -170,6 +175,7 @@ __global__ void encode_residues(uint64_t* out, const double2* __restrict__ v, co
 __global__ void encrypt_prep(uint64_t* U, uint64_t* E1, uint64_t* E2, const uint64_t* __restrict__ m,
                              const int64_t* __restrict__ u, const int64_t* __restrict__ e1,
                              const int64_t* __restrict__ e2, const PrimeConst* __restrict__ pc, unsigned N) {
+  pdl_begin();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   const int l = blockIdx.y;
   if (t >= N) return;
@@ -230,22 +236,19 @@ int aoa_encode(aoa_ctx* c, const double* host_vals, int filled, int empty, uint6
     const unsigned M = (unsigned)(2 * E.N);
     const unsigned tile = (unsigned)std::min<long>(slots, kFftTile);
     for (long len = slots; len > (long)tile; len >>= 1) {
-      fft_stage<true><<<(unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream>>>(v, (unsigned)slots, (unsigned)len,
+      launch_pdl(fft_stage<true>, (unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream, v, (unsigned)slots, (unsigned)len,
                                                                                   E.d_ksi, E.d_rot, M);
       AOA_CHECK_LAUNCH();
-      note_launch();
     }
     if (tile >= 2) {
-      fft_inv_tile<<<(unsigned)(slots / tile), std::min(tile / 2, 1024u), tile * sizeof(double2), C.stream>>>(
+      launch_pdl(fft_inv_tile, (unsigned)(slots / tile), std::min(tile / 2, 1024u), tile * sizeof(double2), C.stream, 
           v, tile, E.d_ksi, E.d_rot, M);
       AOA_CHECK_LAUNCH();
-      note_launch();
     }
     dim3 grid((unsigned)((E.N + 255) / 256), (unsigned)nlimbs);
-    encode_residues<<<grid, 256, 0, C.stream>>>(d_out, v, E.d_pc, (unsigned)E.N, log_size,
+    launch_pdl(encode_residues, grid, 256, 0, C.stream, d_out, v, E.d_pc, (unsigned)E.N, log_size,
                                                  (unsigned)(E.N / 2 / slots), (double)slots, (double)scale);
     AOA_CHECK_LAUNCH();
-    note_launch();
     if (domain != AOA_COEF) xform(E, domain, d_out, 1, 0, nlimbs, nlimbs, true, C.stream);
   });
 }
@@ -273,17 +276,14 @@ int aoa_decode(aoa_ctx* c, const uint64_t* d_m, int domain, int slots, uint64_t 
     }
     const unsigned M = (unsigned)(2 * E.N);
     const unsigned tile = (unsigned)std::min<int>(slots, kFftTile);
-    fft_fwd_tile_from_message<<<(unsigned)(slots / tile), std::max(1u, std::min(tile / 2, 1024u)),
-                                tile * sizeof(double2), C.stream>>>(
+    launch_pdl(fft_fwd_tile_from_message, (unsigned)(slots / tile), std::max(1u, std::min(tile / 2, 1024u)), tile * sizeof(double2), C.stream, 
         v, m0, E.primes[0], (double)scale, log_size, tile, (unsigned)(E.N / 2 / slots), (unsigned)(E.N / 2), E.d_ksi,
         E.d_rot, M);
     AOA_CHECK_LAUNCH();
-    note_launch();
     for (long len = 2L * tile; len <= slots; len <<= 1) {
-      fft_stage<false><<<(unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream>>>(v, (unsigned)slots, (unsigned)len,
+      launch_pdl(fft_stage<false>, (unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream, v, (unsigned)slots, (unsigned)len,
                                                                                    E.d_ksi, E.d_rot, M);
       AOA_CHECK_LAUNCH();
-      note_launch();
     }
     AOA_CUDA(cudaMemcpyAsync(host_vals, v, (size_t)slots * 16, cudaMemcpyDeviceToHost, C.stream));
     AOA_CUDA(cudaStreamSynchronize(C.stream));
@@ -326,9 +326,8 @@ int aoa_encrypt(aoa_ctx* c, aoa_ct* out, const uint64_t* d_m, int m_domain, aoa_
       m = E2;
     }
     dim3 grid((unsigned)((E.N + 255) / 256), (unsigned)E.k);
-    encrypt_prep<<<grid, 256, 0, C.stream>>>(U, E1, E2, m, d_u, d_e1, d_e2, E.d_pc, (unsigned)E.N);
+    launch_pdl(encrypt_prep, grid, 256, 0, C.stream, U, E1, E2, m, d_u, d_e1, d_e2, E.d_pc, (unsigned)E.N);
     AOA_CHECK_LAUNCH();
-    note_launch();
     ntt_batch(E, U, 3, 0, E.k, E.k, true, C.stream);      // U, E1, E2: 3 polys of k limbs
     ct_to_domain(C, pk, AOA_NTT, E.k);
     const long half = (long)E.k * E.N;

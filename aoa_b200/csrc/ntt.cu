@@ -27,6 +27,7 @@ void ntt_init(Engine& E) {
 // the same epilogue as a separate pass over transformed data (small rings)
 __global__ void ntt_epilogue_kernel(const uint64_t* data, long poly_stride, int npolys, int nlimbs, int first_prime,
                                     int prime_shift, const PrimeConst* pc, int log_n, const __grid_constant__ NttEpi e) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long total = (long)npolys * nlimbs * N;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -42,6 +43,7 @@ __global__ void ntt_epilogue_kernel(const uint64_t* data, long poly_stride, int 
 // memory, one radix-2 stage per step, canonical (strict) butterflies with the
 // same merged tables as the large kernels.
 __global__ void ntt_small(NttBatch b, bool fwd) {
+  pdl_begin();
   extern __shared__ __align__(16) uint64_t xs[];
   const int N = 1 << b.log_n;
   for (int j = blockIdx.x; j < b.nitems; j += gridDim.x) {
@@ -152,11 +154,10 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
     b.nitems = npolys * nlimbs;
     b.data = data;
     const int grid = std::min(b.nitems, 8 * E.num_sms);
-    ntt_small<<<grid, std::max(32, std::min((int)n / 2, 256)), n * 8, st>>>(b, forward);
-    note_launch();
+    launch_pdl(ntt_small, grid, std::max(32, std::min((int)n / 2, 256)), n * 8, st, b, forward);
     if (epi.mode != kEpiStore) {
-      ntt_epilogue_kernel<<<2 * E.num_sms, 256, 0, st>>>(data, poly_stride, npolys, nlimbs, first_prime, T.prime_shift, T.pc, T.log_n, epi);
-      note_launch();
+      launch_pdl(ntt_epilogue_kernel, 2 * E.num_sms, 256, 0, st, data, poly_stride, npolys, nlimbs, first_prime,
+                                                         T.prime_shift, T.pc, T.log_n, epi);
     }
     AOA_CHECK_LAUNCH();
     return;

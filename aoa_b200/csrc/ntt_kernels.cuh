@@ -472,7 +472,8 @@ ntt_cols(NttBatch b, const __grid_constant__ CUtensorMap tmap) {
     for (int e = threadIdx.x; e < D::S; e += blockDim.x) tws[tb * D::S + e] = tw[e];
     cur_limb = limb;
   };
-  if (j_lo < j_hi) twiddles(j_lo / b.npolys);
+  if (j_lo < j_hi) twiddles(j_lo / b.npolys);   // a constant table: fetched while the previous kernel ends
+  pdl_begin();
   if (j_lo < j_hi) issue(j_lo, 0);
   for (int j = j_lo, it = 0; j < j_hi; j++, it++) {
     const int bi = it & 1;
@@ -592,6 +593,7 @@ ntt_cols_wo(NttBatch b) {
   __syncthreads();
   const int j_lo = (int)((long)blockIdx.y * b.nitems / G), j_hi = (int)((long)(blockIdx.y + 1) * b.nitems / G);
   auto prime_of = [&](int j) { return b.first_prime + ((j / b.npolys) >> b.prime_shift); };
+  pdl_begin();
   if (warp == NW) {
     // producer: tile rows of W words (one bulk copy each) and, when the prime
     // of the buffer changes, its S twiddles
@@ -754,7 +756,8 @@ ntt_rows(NttBatch b, const __grid_constant__ NttEpi epi) {
     q = b.pc[prime].q;
     cur_limb = limb;
   };
-  if (j_lo < j_hi) twiddles(j_lo / b.npolys);
+  if (j_lo < j_hi) twiddles(j_lo / b.npolys);   // a constant table: fetched while the previous kernel ends
+  pdl_begin();
   if (threadIdx.x == 0 && j_lo < j_hi) issue(j_lo, 0);
   for (int j = j_lo, it = 0; j < j_hi; j++, it++) {
     const int bi = it & 1;
@@ -903,9 +906,8 @@ static void launch_cols(const Engine& E, const NttBatch& b0, bool fwd, cudaStrea
   // a tensor-map tile load needs the rows of the tile in order (no row swizzle: W = 16)
   b.use_tma = E.tune.ntt_cols_tma && Tl::W == 16 && col_tensor_map(b, Tl::W, &map) ? 1 : 0;
   dim3 grid(C / Tl::W, ctas_per_tile(E, C / Tl::W, b.nitems, Tl::MIN_BLOCKS));
-  if (fwd) ntt_cols<LOG_R, DIV, LAZY, true><<<grid, Tl::THREADS, Tl::SMEM, st>>>(b, map);
-  else ntt_cols<LOG_R, DIV, LAZY, false><<<grid, Tl::THREADS, Tl::SMEM, st>>>(b, map);
-  note_launch();
+  if (fwd) launch_pdl(ntt_cols<LOG_R, DIV, LAZY, true>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
+  else launch_pdl(ntt_cols<LOG_R, DIV, LAZY, false>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
 }
 
 template <int LOG_R, int NW>
@@ -914,9 +916,8 @@ static void launch_cols_wo(const Engine& E, const NttBatch& b, bool fwd, cudaStr
   const int C = 1 << b.log_c;
   if (C % Tl::W) throw AoaError(AOA_ERR_BAD_PARAM, "ntt: column tile does not divide C");
   dim3 grid(C / Tl::W, ctas_per_tile(E, C / Tl::W, b.nitems, Tl::MIN_BLOCKS));
-  if (fwd) ntt_cols_wo<LOG_R, NW, true><<<grid, Tl::THREADS, Tl::SMEM, st>>>(b);
-  else ntt_cols_wo<LOG_R, NW, false><<<grid, Tl::THREADS, Tl::SMEM, st>>>(b);
-  note_launch();
+  if (fwd) launch_pdl(ntt_cols_wo<LOG_R, NW, true>, grid, Tl::THREADS, Tl::SMEM, st, b);
+  else launch_pdl(ntt_cols_wo<LOG_R, NW, false>, grid, Tl::THREADS, Tl::SMEM, st, b);
 }
 
 template <int LOG_C, int DIV, int LAZY>
@@ -925,9 +926,8 @@ static void launch_rows(const Engine& E, const NttBatch& b, bool fwd, cudaStream
   const int R = 1 << b.log_r;
   if (R % Tl::ROWS) throw AoaError(AOA_ERR_BAD_PARAM, "ntt: row tile does not divide R");
   dim3 grid(R / Tl::ROWS, ctas_per_tile(E, R / Tl::ROWS, b.nitems, Tl::MIN_BLOCKS));
-  if (fwd) ntt_rows<LOG_C, DIV, LAZY, true><<<grid, Tl::THREADS, Tl::SMEM, st>>>(b, epi);
-  else ntt_rows<LOG_C, DIV, LAZY, false><<<grid, Tl::THREADS, Tl::SMEM, st>>>(b, epi);
-  note_launch();
+  if (fwd) launch_pdl(ntt_rows<LOG_C, DIV, LAZY, true>, grid, Tl::THREADS, Tl::SMEM, st, b, epi);
+  else launch_pdl(ntt_rows<LOG_C, DIV, LAZY, false>, grid, Tl::THREADS, Tl::SMEM, st, b, epi);
 }
 
 #define AOA_NTT_SIZES(X) X(5) X(6) X(7) X(8) X(9) X(10)

@@ -7,6 +7,7 @@
 // the prime of limb l is prime0 + l.  Every limb is N contiguous words, so each
 // warp reads and writes 256 contiguous bytes per operand.
 #include "aoa_internal.h"
+#include "async.cuh"
 
 namespace aoa {
 
@@ -29,6 +30,7 @@ __device__ __forceinline__ long coef_u(int u) { return ((long)blockIdx.x * kEwPe
 
 // c = a (op) b over limbs; op: 0 add, 1 sub, 2 mul (Montgomery pair), 3 neg(a)
 __global__ void ew_binary(Limbs c, CLimbs a, CLimbs b, int op, int prime0, const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long off = (long)blockIdx.y * N + coef_index();
   const PrimeConst& P = pc[prime0 + blockIdx.y];
@@ -47,6 +49,7 @@ __global__ void ew_binary(Limbs c, CLimbs a, CLimbs b, int op, int prime0, const
 // op: 0 add, 1 sub, 2 mul
 __global__ void ew_scalar(Limbs c, CLimbs a, const uint64_t* s, int op, int prime0, const PrimeConst* pc,
                           int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long off = (long)blockIdx.y * N + coef_index();
   const PrimeConst& P = pc[prime0 + blockIdx.y];
@@ -57,6 +60,7 @@ __global__ void ew_scalar(Limbs c, CLimbs a, const uint64_t* s, int op, int prim
 
 // d = a * b + c  (ntt_vector_seqop)
 __global__ void ew_muladd(Limbs d, CLimbs a, CLimbs b, CLimbs c, int prime0, const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long off = (long)blockIdx.y * N + coef_index();
   const PrimeConst& P = pc[prime0 + blockIdx.y];
@@ -116,6 +120,7 @@ __device__ __forceinline__ void tensor_ew(const uint64_t* a, long a_half, const 
 
 __global__ void hmult_tensor(const uint64_t* a, const uint64_t* b, long a_half, long b_half, uint64_t* d0,
                              uint64_t* d1, uint64_t* d2, const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long limb = (long)blockIdx.y << log_n;
   const PrimeConst P = pc[blockIdx.y];
   tensor_ew(a + limb, a_half, b + limb, b_half, d0 + limb, d1 + limb, d2 + limb, P);
@@ -127,6 +132,7 @@ __global__ void hmult_tensor(const uint64_t* a, const uint64_t* b, long a_half, 
 // the key is [b | a], each (k + kl) limbs in the reference's QB layout.
 __global__ void keyswitch_mul(const uint64_t* xq, const uint64_t* xb, const uint64_t* key, long key_half,
                               uint64_t* k0, uint64_t* k1, int nq, int K, const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const int l = blockIdx.y;
   const int prime = l < nq ? l : K + (l - nq);
@@ -153,6 +159,7 @@ __global__ void keyswitch_mul(const uint64_t* xq, const uint64_t* xb, const uint
 // negacyclic sign (execute_rotation, encoder.cu:300-322).
 __global__ void automorph_coef(uint64_t* out, const uint64_t* in, long poly_stride, long galois,
                                const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long c = coef_index();
   const long off = blockIdx.z * poly_stride + (long)blockIdx.y * N;
@@ -166,6 +173,7 @@ __global__ void automorph_coef(uint64_t* out, const uint64_t* in, long poly_stri
 // psi^(2 br(p) + 1) -> psi^((2 br(p) + 1) g).  Output position p reads the
 // input position holding the evaluation at psi^((2 br(p)+1) g).
 __global__ void automorph_ntt(uint64_t* out, const uint64_t* in, long poly_stride, long galois, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long p = coef_index();
   const long off = blockIdx.z * poly_stride + (long)blockIdx.y * N;
@@ -182,6 +190,7 @@ __global__ void automorph_ntt(uint64_t* out, const uint64_t* in, long poly_strid
 // (poly blockIdx.z % 2, stride half) into out: poly 0 of every op first
 // (op stride half), then poly 1 (block offset n*half).
 __global__ void automorph_ntt_batch(CtPtrs ptr, long half, uint64_t* out, int n, GaloisList gl, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long p = coef_index();
   const int z = blockIdx.z >> 1, poly = blockIdx.z & 1;
@@ -195,6 +204,7 @@ __global__ void automorph_ntt_batch(CtPtrs ptr, long half, uint64_t* out, int n,
 // tensor for op z = blockIdx.z: a = ptr.a[z], b = ptr.b[z] ([c0 | c1], stride half);
 // outputs to the blocks D0 = D, D1 = D + n*half, D2 = D + 2n*half, op stride half.
 __global__ void hmult_tensor_batch(CtPtrs ptr, long half, uint64_t* D, int n, const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const int z = blockIdx.z;
   const long limb = (long)blockIdx.y << log_n;
   const PrimeConst P = pc[blockIdx.y];
@@ -211,6 +221,7 @@ __global__ void hmult_tensor_batch(CtPtrs ptr, long half, uint64_t* D, int n, co
 __global__ void keyswitch_mul_batch(const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
                                     const uint64_t* key, long key_half, uint64_t* k, long k_stride, int n, int nq,
                                     int K, const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const int l = blockIdx.y;
   const int prime = l < nq ? l : K + (l - nq);
@@ -244,6 +255,7 @@ __global__ void keyswitch_mul_batch(const uint64_t* xq, long xq_stride, const ui
 __global__ void keyswitch_mul_keys(const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
                                    KeyPtrs keys, long key_half, uint64_t* k, long k_stride, int n, int nq, int K,
                                    const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const int l = blockIdx.y;
   const int prime = l < nq ? l : K + (l - nq);
@@ -278,36 +290,35 @@ static dim3 ew4_grid(const Engine& E, int nlimbs, int npolys) { return dim3(E.N 
 void ew_binary_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* b, long bs,
                   int op, int prime0, int nlimbs, int npolys, cudaStream_t st) {
   if (nlimbs <= 0 || npolys <= 0) return;
-  ew_binary<<<ew_grid(E, nlimbs, npolys), 256, 0, st>>>(Limbs{c, cs}, CLimbs{a, as}, CLimbs{b, bs}, op, prime0,
-                                                        E.d_pc, E.log_n); note_launch();
+  launch_pdl(ew_binary, ew_grid(E, nlimbs, npolys), 256, 0, st, Limbs{c, cs}, CLimbs{a, as}, CLimbs{b, bs}, op, prime0,
+                                                        E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
 void ew_scalar_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* d_scalars,
                   int op, int prime0, int nlimbs, int npolys, cudaStream_t st) {
   if (nlimbs <= 0 || npolys <= 0) return;
-  ew_scalar<<<ew_grid(E, nlimbs, npolys), 256, 0, st>>>(Limbs{c, cs}, CLimbs{a, as}, d_scalars, op, prime0,
-                                                        E.d_pc, E.log_n); note_launch();
+  launch_pdl(ew_scalar, ew_grid(E, nlimbs, npolys), 256, 0, st, Limbs{c, cs}, CLimbs{a, as}, d_scalars, op, prime0,
+                                                        E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
 void ew_muladd_op(const Engine& E, uint64_t* d, long ds, const uint64_t* a, long as, const uint64_t* b, long bs,
                   const uint64_t* c, long cs, int prime0, int nlimbs, int npolys, cudaStream_t st) {
   if (nlimbs <= 0 || npolys <= 0) return;
-  ew_muladd<<<ew_grid(E, nlimbs, npolys), 256, 0, st>>>(Limbs{d, ds}, CLimbs{a, as}, CLimbs{b, bs},
-                                                        CLimbs{c, cs}, prime0, E.d_pc, E.log_n); note_launch();
+  launch_pdl(ew_muladd, ew_grid(E, nlimbs, npolys), 256, 0, st, Limbs{d, ds}, CLimbs{a, as}, CLimbs{b, bs},
+                                                        CLimbs{c, cs}, prime0, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
 void tensor_op(const Engine& E, const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0,
                uint64_t* d1, uint64_t* d2, int nlimbs, cudaStream_t st) {
-  hmult_tensor<<<ew4_grid(E, nlimbs, 1), 256, 0, st>>>(a, b, a_half, b_half, d0, d1, d2, E.d_pc, E.log_n); note_launch();
+  launch_pdl(hmult_tensor, ew4_grid(E, nlimbs, 1), 256, 0, st, a, b, a_half, b_half, d0, d1, d2, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
 void tensor_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D, int n, int nlimbs, cudaStream_t st) {
-  hmult_tensor_batch<<<ew4_grid(E, nlimbs, n), 256, 0, st>>>(ptr, half, D, n, E.d_pc, E.log_n);
-  note_launch();
+  launch_pdl(hmult_tensor_batch, ew4_grid(E, nlimbs, n), 256, 0, st, ptr, half, D, n, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
@@ -315,9 +326,8 @@ void keyswitch_mul_batch_op(const Engine& E, const uint64_t* xq, long xq_stride,
                             const uint64_t* key, uint64_t* k, long k_stride, int n, int nq, cudaStream_t st, int nb) {
   const long half = (long)E.nprimes * E.N;
   if (nb < 0) nb = E.kl;
-  keyswitch_mul_batch<<<ew4_grid(E, nq + nb, 1), 256, 0, st>>>(xq, xq_stride, xb, xb_stride, key, half, k, k_stride,
+  launch_pdl(keyswitch_mul_batch, ew4_grid(E, nq + nb, 1), 256, 0, st, xq, xq_stride, xb, xb_stride, key, half, k, k_stride,
                                                                n, nq, E.k, E.d_pc, E.log_n);
-  note_launch();
   AOA_CHECK_LAUNCH();
 }
 
@@ -325,35 +335,33 @@ void keyswitch_mul_op(const Engine& E, const uint64_t* xq, const uint64_t* xb, c
                       uint64_t* k1, int nq, cudaStream_t st, int nb) {
   const long half = (long)E.nprimes * E.N;
   if (nb < 0) nb = E.kl;
-  keyswitch_mul<<<ew4_grid(E, nq + nb, 1), 256, 0, st>>>(xq, xb, key, half, k0, k1, nq, E.k, E.d_pc, E.log_n); note_launch();
+  launch_pdl(keyswitch_mul, ew4_grid(E, nq + nb, 1), 256, 0, st, xq, xb, key, half, k0, k1, nq, E.k, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
 void automorph_coef_op(const Engine& E, uint64_t* out, const uint64_t* in, long poly_stride, long galois,
                        int nlimbs, int npolys, cudaStream_t st) {
-  automorph_coef<<<ew_grid(E, nlimbs, npolys), 256, 0, st>>>(out, in, poly_stride, galois, E.d_pc, E.log_n); note_launch();
+  launch_pdl(automorph_coef, ew_grid(E, nlimbs, npolys), 256, 0, st, out, in, poly_stride, galois, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
 void automorph_ntt_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* out, int n,
                             const GaloisList& galois, int nlimbs, cudaStream_t st) {
-  automorph_ntt_batch<<<ew_grid(E, nlimbs, 2 * n), 256, 0, st>>>(ptr, half, out, n, galois, E.log_n);
-  note_launch();
+  launch_pdl(automorph_ntt_batch, ew_grid(E, nlimbs, 2 * n), 256, 0, st, ptr, half, out, n, galois, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
 void keyswitch_mul_keys_op(const Engine& E, const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
                            const KeyPtrs& keys, uint64_t* k, long k_stride, int n, int nq, cudaStream_t st) {
   const long half = (long)E.nprimes * E.N;
-  keyswitch_mul_keys<<<ew4_grid(E, nq + E.kl, 1), 256, 0, st>>>(xq, xq_stride, xb, xb_stride, keys, half, k, k_stride,
+  launch_pdl(keyswitch_mul_keys, ew4_grid(E, nq + E.kl, 1), 256, 0, st, xq, xq_stride, xb, xb_stride, keys, half, k, k_stride,
                                                                  n, nq, E.k, E.d_pc, E.log_n);
-  note_launch();
   AOA_CHECK_LAUNCH();
 }
 
 void automorph_ntt_op(const Engine& E, uint64_t* out, const uint64_t* in, long poly_stride, long galois,
                       int nlimbs, int npolys, cudaStream_t st) {
-  automorph_ntt<<<ew_grid(E, nlimbs, npolys), 256, 0, st>>>(out, in, poly_stride, galois, E.log_n); note_launch();
+  launch_pdl(automorph_ntt, ew_grid(E, nlimbs, npolys), 256, 0, st, out, in, poly_stride, galois, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 

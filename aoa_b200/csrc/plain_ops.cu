@@ -5,6 +5,7 @@
 // reference's inner products and of the logistic-regression steps its
 // downstream user runs.  Scale bookkeeping follows the reference exactly.
 #include "aoa_internal.h"
+#include "async.cuh"
 
 using namespace aoa;
 
@@ -25,6 +26,7 @@ struct LimbScalars {
 // (the real plane of a DGT limb).
 __global__ void scalar_limb_op(uint64_t* out, const uint64_t* in, long poly_stride, LimbScalars s, int op,
                                const PrimeConst* __restrict__ pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= N) return;
@@ -42,8 +44,7 @@ void scalar_op(Ctx& C, uint64_t* out, const uint64_t* in, long poly_stride, int 
                const LimbScalars& s, int op) {
   const Engine& E = *C.E;
   dim3 grid((unsigned)((E.N + 255) / 256), (unsigned)nlimbs, (unsigned)npolys);
-  scalar_limb_op<<<grid, 256, 0, C.stream>>>(out, in, poly_stride, s, op, E.d_pc, E.log_n);
-  note_launch();
+  launch_pdl(scalar_limb_op, grid, 256, 0, C.stream, out, in, poly_stride, s, op, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 

@@ -78,6 +78,7 @@ __device__ __forceinline__ void conv_store(const ConvArgs& a, int jj, uint64_t r
 
 __global__ void __launch_bounds__(kConvThreads, 2)
 basis_convert(ConvArgs a, int j_first, int j_end) {
+  pdl_begin();
   extern __shared__ uint64_t smat[];    // [nin][kConvOut]
   const int nout = min(kConvOut, j_end - j_first);
   for (int e = threadIdx.x; e < a.nin * kConvOut; e += blockDim.x) {
@@ -357,6 +358,7 @@ basis_convert_tc(ConvArgs a, int j_first, int j_end) {
     }
     if (MODE >= kRescaleTop) dv_next = a.d[poly * a.d_poly_stride + c0 + erow];
   };
+  pdl_begin();                                             // everything above reads constants only
   if (blockIdx.x < ntiles) load_inputs(blockIdx.x);
   bool ok = __syncthreads_and(mbar_wait(&mbar[0], 0, a.spin));
   bool in_flight = false;                                  // an MMA group not yet waited for
@@ -482,9 +484,7 @@ static void run_convert(const Engine& E, const ConvArgs& a, int npolys, int j_be
     bool q1 = true;                               // every input and output prime q = 1 mod 2^32 below 2^60
     for (int i = 0; i < a.nin; i++) q1 = q1 && E.prime_kind[a.in_prime0 + i] == kButterflyLazyQ1;
     for (int j = 0; j < j_end; j++) q1 = q1 && E.prime_kind[a.out_prime0 + j] == kButterflyLazyQ1;
-#define AOA_TC(M)                                                                                   \
-  if (q1) basis_convert_tc<M, true><<<grid_tc, kTcThreads, kTcSmem, st>>>(t, j_begin, j_end);     \
-  else basis_convert_tc<M, false><<<grid_tc, kTcThreads, kTcSmem, st>>>(t, j_begin, j_end);
+#define AOA_TC(M) launch_pdl(q1 ? basis_convert_tc<M, true> : basis_convert_tc<M, false>, grid_tc, kTcThreads, kTcSmem, st, t, j_begin, j_end);
     switch (a.mode) {
       case kRaw: AOA_TC(kRaw) break;
       case kModDown: AOA_TC(kModDown) break;
@@ -493,13 +493,11 @@ static void run_convert(const Engine& E, const ConvArgs& a, int npolys, int j_be
       default: AOA_TC(kRescaleFused) break;
     }
 #undef AOA_TC
-    note_launch();
     AOA_CHECK_LAUNCH();
     return;
   }
   for (int j0 = j_begin; j0 < j_end; j0 += kConvOut) {
-    basis_convert<<<grid, kConvThreads, smem, st>>>(a, j0, j_end);
-    note_launch();
+    launch_pdl(basis_convert, grid, kConvThreads, smem, st, a, j0, j_end);
   }
   AOA_CHECK_LAUNCH();
 }
@@ -601,6 +599,7 @@ void rescale_corrections(const Engine& E, const uint64_t* in_b, long in_stride, 
 // npolys polys (stride poly_stride) in place, coefficient domain.
 __global__ void rescale_kernel(uint64_t* d, long poly_stride, int level, const ShoupW* inv,
                                const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y;
@@ -613,9 +612,8 @@ __global__ void rescale_kernel(uint64_t* d, long poly_stride, int level, const S
 void rescale(const Engine& E, uint64_t* d, long poly_stride, int npolys, int level, cudaStream_t st) {
   if (level < 1 || level >= E.k) throw AoaError(AOA_ERR_LEVEL_EXHAUSTED, "rescale: level must be >= 1");
   dim3 grid(E.N / 256, level, npolys);
-  rescale_kernel<<<grid, 256, 0, st>>>(d, poly_stride, level, E.rns.resc_inv + (long)level * E.k, E.d_pc,
+  launch_pdl(rescale_kernel, grid, 256, 0, st, d, poly_stride, level, E.rns.resc_inv + (long)level * E.k, E.d_pc,
                                        E.log_n);
-  note_launch();
   AOA_CHECK_LAUNCH();
 }
 
@@ -639,6 +637,7 @@ __global__ void ks_combine_kernel(uint64_t* out, long out_stride, const uint64_t
                                   const uint64_t* k, long k_stride, const uint64_t* y, long y_stride,
                                   const ShoupW* binv, const ShoupW* resc, const PrimeConst* pc, int prime0,
                                   int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const int i = prime0 + blockIdx.y, p = blockIdx.z;
   const long limb = (long)blockIdx.y * N;
@@ -667,6 +666,7 @@ __global__ void ks_combine_kernel(uint64_t* out, long out_stride, const uint64_t
 __global__ void ks_combine_ptr_kernel(OutPtrs outp, const uint64_t* base, long base_stride, int base_polys,
                                       const uint64_t* k, long k_stride, const uint64_t* y, long y_stride,
                                       const ShoupW* binv, const ShoupW* resc, const PrimeConst* pc, int log_n) {
+  pdl_begin();
   const long N = 1L << log_n;
   const int i = blockIdx.y, p = blockIdx.z;
   const long limb = (long)i * N;
@@ -697,9 +697,8 @@ void ks_combine_ptr(const Engine& E, const OutPtrs& outp, const uint64_t* base, 
   if (nlimbs <= 0) return;
   dim3 grid(E.N / (256 * kCombPer), nlimbs, npolys);
   const ShoupW* resc = rescale_level > 0 ? E.rns.resc_inv + (long)rescale_level * E.k : nullptr;
-  ks_combine_ptr_kernel<<<grid, 256, 0, st>>>(outp, base, base_stride, base_polys < 0 ? npolys : base_polys, k,
+  launch_pdl(ks_combine_ptr_kernel, grid, 256, 0, st, outp, base, base_stride, base_polys < 0 ? npolys : base_polys, k,
                                               k_stride, y, y_stride, E.rns.moddown_binv, resc, E.d_pc, E.log_n);
-  note_launch();
   AOA_CHECK_LAUNCH();
 }
 
@@ -709,9 +708,8 @@ void ks_combine(const Engine& E, uint64_t* out, long out_stride, const uint64_t*
   if (nlimbs <= 0) return;
   dim3 grid(E.N / (256 * kCombPer), nlimbs, npolys);
   const ShoupW* resc = rescale_level > 0 ? E.rns.resc_inv + (long)rescale_level * E.k : nullptr;
-  ks_combine_kernel<<<grid, 256, 0, st>>>(out, out_stride, base, base_stride, k, k_stride, y, y_stride,
+  launch_pdl(ks_combine_kernel, grid, 256, 0, st, out, out_stride, base, base_stride, k, k_stride, y, y_stride,
                                           E.rns.moddown_binv, resc, E.d_pc, prime0, E.log_n);
-  note_launch();
   AOA_CHECK_LAUNCH();
 }
 
