@@ -347,6 +347,14 @@ void keyswitch_mul_batch_op(const Engine& E, const uint64_t* xq, long xq_stride,
 void ks_combine_ptr(const Engine& E, const OutPtrs& outp, const uint64_t* base, long base_stride, const uint64_t* k,
                     long k_stride, const uint64_t* y, long y_stride, int nlimbs, int npolys, int rescale_level,
                     cudaStream_t st, int base_polys = -1);
+// ks_finish.cu: the Q limbs of a key switch in one pass over the operands
+void tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, int n, int nlimbs, cudaStream_t st);
+void hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key, uint64_t* U,
+                  int n, int level, cudaStream_t st);
+void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+                     const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
+void galois_finish_op(const Engine& E, const uint64_t* R, long half, const KeyPtrs& keys, bool one_key,
+                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, cudaStream_t st);
 void automorph_ntt_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* out, int n,
                             const GaloisList& galois, int nlimbs, cudaStream_t st);
 // key products with a key per op (keys.k[z], [b | a] over all primes)

@@ -47,7 +47,7 @@ Workspace carve(const Engine& E, uint64_t* p) {
   return w;
 }
 
-static Workspace get_ws(Ctx& C) {
+static uint64_t* get_scratch(Ctx& C) {
   const size_t need = workspace_words(*C.E) * sizeof(uint64_t);
   if (C.scratch_bytes < need) {
     if (C.scratch) AOA_CUDA(cudaFreeAsync(C.scratch, C.stream));
@@ -60,7 +60,7 @@ static Workspace get_ws(Ctx& C) {
     }
     C.scratch_bytes = need;
   }
-  return carve(*C.E, (uint64_t*)C.scratch);
+  return (uint64_t*)C.scratch;
 }
 
 // Limb transforms of the given kind (AOA_NTT: negacyclic NTT of aoa-ntt;
@@ -85,15 +85,6 @@ static void to_domain(Ctx& C, aoa_ct* ct, int domain, int nlimbs) { ct_to_domain
 static void copy_limbs(Ctx& C, uint64_t* dst, const uint64_t* src, long words) {
   AOA_CUDA(cudaMemcpyAsync(dst, src, (size_t)words * 8, cudaMemcpyDeviceToDevice, C.stream));
 }
-
-// Key-switch core on the Q limbs 0..level of x, given in both domains
-// (x_coef, x_ntt).  Leaves in w.KS = [x*b | x*a] (stride k + kl limbs): the Q
-// limbs in the transform domain, the kl B limbs back in coefficients.
-// (ModUp poly_modup, key products poly_mul, ckks.cpp:309-314.)
-// Fused transform ends (out-of-place inverse, key products, key-switch
-// combine; engine knob "fuse", a bit mask) on NTT contexts; DGT contexts take
-// the separate kernels.
-static bool fused(const Ctx& C, int what) { return C.transform == AOA_NTT && (C.E->tune.fuse & what); }
 
 // Forward transform of the corrections Y (npolys polys of stride k limbs,
 // limbs 0..nlimbs-1) with the key-switch combine as its epilogue.
@@ -120,31 +111,21 @@ static void combine_into(Ctx& C, uint64_t* Y, int npolys, int nlimbs, const uint
   ntt_batch_io(E, Y, npolys, 0, nlimbs, E.k, true, io, st ? st : C.stream);
 }
 
-static void keyswitch_core(Ctx& C, const Workspace& w, const uint64_t* x_coef, const uint64_t* x_ntt,
+// Key switch of a DGT context's automorphisms, on the Q limbs 0..level of x,
+// given in both domains (x_coef, x_dgt).  Leaves in w.KS = [x*b | x*a] (stride
+// k + kl limbs): the Q limbs in the transform domain, the kl B limbs back in
+// coefficients.  (ModUp poly_modup, key products poly_mul, ckks.cpp:309-314.)
+static void keyswitch_core(Ctx& C, const Workspace& w, const uint64_t* x_coef, const uint64_t* x_dgt,
                            const aoa_swk* key, int level) {
   const Engine& E = *C.E;
   const long N = E.N;
   const int m = level + 1;
-  const int tk = C.transform;
-  if (key->domain != tk) throw AoaError(AOA_ERR_BAD_PARAM, "the switching key is in another transform domain");
+  if (key->domain != AOA_DGT) throw AoaError(AOA_ERR_BAD_PARAM, "the switching key is in another transform domain");
   modup(E, x_coef, 0, w.UB, 0, 1, level, C.stream);
   const long ks = (long)(E.k + E.kl) * N;
-  if (fused(C, kFuseKeyProduct)) {
-    // forward transform of the special limbs with the key products as its epilogue
-    NttIo io;
-    io.epi.mode = kEpiKeyProduct;
-    io.epi.out = w.KS + (long)m * N;
-    io.epi.out_poly1 = ks;
-    io.epi.key = key->d;
-    io.epi.key_half = (long)E.nprimes * N;
-    ntt_batch_io(E, w.UB, 1, E.k, E.kl, E.kl, true, io, C.stream);
-    keyswitch_mul_op(E, x_ntt, nullptr, key->d, w.KS, w.KS + ks, m, C.stream, 0);
-  } else {
-    xform(E, tk, w.UB, 1, E.k, E.kl, E.kl, true, C.stream);
-    if (tk == AOA_DGT) gi_keyswitch_mul_op(E, x_ntt, w.UB, key->d, w.KS, w.KS + ks, m, C.stream);
-    else keyswitch_mul_op(E, x_ntt, w.UB, key->d, w.KS, w.KS + ks, m, C.stream);
-  }
-  xform(E, tk, w.KS + (long)m * N, 2, E.k, E.kl, E.k + E.kl, false, C.stream);
+  xform(E, AOA_DGT, w.UB, 1, E.k, E.kl, E.kl, true, C.stream);
+  gi_keyswitch_mul_op(E, x_dgt, w.UB, key->d, w.KS, w.KS + ks, m, C.stream);
+  xform(E, AOA_DGT, w.KS + (long)m * N, 2, E.k, E.kl, E.k + E.kl, false, C.stream);
 }
 
 static uint64_t scale_after_mult(const Engine& E, uint64_t sa, uint64_t sb, int level) {
@@ -152,98 +133,17 @@ static uint64_t scale_after_mult(const Engine& E, uint64_t sa, uint64_t sb, int 
   return (uint64_t)(p / E.primes[level]);
 }
 
-// Finishes a key switch whose products sit in w.KS and writes the transform
-// domain result to out (2 polys of stride `half`):
-//   rescale:  out = Rescale(base + ModDown(KS))   (limbs 0..level-1)
-//   else:     out = base + ModDown(KS)            (limbs 0..level)
-// base = [b0 | b1] (stride `half`, transform domain) or b1 == nullptr (zero).
-static void keyswitch_finish(Ctx& C, const Workspace& w, uint64_t* out, long half, const uint64_t* b0,
-                             const uint64_t* b1, int level, bool do_rescale) {
+// Finishes it: out = base + ModDown(KS) (limbs 0..level, transform domain) with
+// the base in poly 0 only.
+static void keyswitch_finish(Ctx& C, const Workspace& w, uint64_t* out, long half, const uint64_t* base, int level) {
   const Engine& E = *C.E;
   const long N = E.N;
   const int m = level + 1;
   const long ks_stride = (long)(E.k + E.kl) * N;
-  const uint64_t* kb = w.KS + (long)m * N;
-  if (do_rescale) {
-    // u_l = limb l of (base + k B^-1) in coefficients, for both polys
-    uint64_t* U = w.L4;
-    if (b0 && b1 == b0 + half) {
-      ks_combine(E, U, N, b0 + (long)level * N, half, w.KS + (long)level * N, ks_stride, nullptr, 0, 1, 2, 0,
-                 C.stream, level);
-    } else {
-      ks_combine(E, U, 0, b0 ? b0 + (long)level * N : nullptr, 0, w.KS + (long)level * N, 0, nullptr, 0, 1, 1,
-                 0, C.stream, level);
-      ks_combine(E, U + N, 0, b1 ? b1 + (long)level * N : nullptr, 0, w.KS + ks_stride + (long)level * N, 0,
-                 nullptr, 0, 1, 1, 0, C.stream, level);
-    }
-    xform(E, C.transform, U, 2, level, 1, 1, false, C.stream);
-    rescale_corrections(E, kb, ks_stride, U, N, w.CL, N, w.Y, (long)E.k * N, 2, level, C.stream);
-    if (fused(C, kFuseCombine) && (!b1 || b1 == b0 + half)) {
-      combine_into(C, w.Y, 2, level, b0, half, b1 ? 2 : 1, w.KS, ks_stride, level, out, half, nullptr);
-      return;
-    }
-    xform(E, C.transform, w.Y, 2, 0, level, E.k, true, C.stream);
-    if (b0 && b1 == b0 + half) {
-      ks_combine(E, out, half, b0, half, w.KS, ks_stride, w.Y, (long)E.k * N, level, 2, level, C.stream);
-    } else {
-      ks_combine(E, out, 0, b0, 0, w.KS, 0, w.Y, 0, level, 1, level, C.stream);
-      ks_combine(E, out + half, 0, b1, 0, w.KS + ks_stride, 0, w.Y + (long)E.k * N, 0, level, 1, level, C.stream);
-    }
-  } else {
-    moddown_conv(E, kb, ks_stride, w.Y, (long)E.k * N, 2, m, C.stream);
-    if (fused(C, kFuseCombine) && (!b1 || b1 == b0 + half)) {
-      combine_into(C, w.Y, 2, m, b0, half, b1 ? 2 : 1, w.KS, ks_stride, 0, out, half, nullptr);
-      return;
-    }
-    xform(E, C.transform, w.Y, 2, 0, m, E.k, true, C.stream);
-    if (b0 && b1 == b0 + half) {
-      ks_combine(E, out, half, b0, half, w.KS, ks_stride, w.Y, (long)E.k * N, m, 2, 0, C.stream);
-    } else {
-      ks_combine(E, out, 0, b0, 0, w.KS, 0, w.Y, 0, m, 1, 0, C.stream);
-      ks_combine(E, out + half, 0, b1, 0, w.KS + ks_stride, 0, w.Y + (long)E.k * N, 0, m, 1, 0, C.stream);
-    }
-  }
-}
-
-// HMult + relinearisation (ckks_mul_without_rescale, ckks.cpp:273-332),
-// optionally followed by the rescale of ckks_mul (ckks.cpp:334-347).
-// Transform-domain pipeline: tensor, one inverse transform of d2 for ModUp,
-// the key products, inverse transforms of their B limbs only, and ModDown
-// merged with the rescale (one forward transform per output limb).  The
-// result is left in the transform domain (the reference leaves coefficients;
-// the residues of every live limb are the same after a domain change).
-static void hmult_core(Ctx& C, const Workspace& w, aoa_ct* out, aoa_ct* a, aoa_ct* b, const aoa_swk* evk,
-                       bool do_rescale) {
-  const Engine& E = *C.E;
-  const long N = E.N;
-  const int level = std::min(a->level, b->level);
-  const int m = level + 1;
-  const long half = (long)E.k * N;
-  // operands to the transform domain, in place (poly_mul does the same, poly_t.cpp:201-220)
-  const int tk = C.transform;
-  to_domain(C, a, tk, a->level + 1);
-  if (b != a) to_domain(C, b, tk, b->level + 1);
-  uint64_t* D0 = w.D;
-  uint64_t* D2 = w.D + 2 * half;
-  if (tk == AOA_DGT) gi_tensor_op(E, a->d, half, b->d, half, D0, D0 + half, D2, m, C.stream);
-  else tensor_op(E, a->d, half, b->d, half, D0, D0 + half, D2, m, C.stream);
-  const uint64_t sa = a->scale, sb = b->scale;
-  const int slots = a->slots;
-  if (fused(C, kFuseSource)) {
-    NttIo io;                                  // inverse of d2 read in place of a copy
-    io.src = D2;
-    io.src_poly_stride = m;
-    ntt_batch_io(E, w.T, 1, 0, m, m, false, io, C.stream);
-  } else {
-    copy_limbs(C, w.T, D2, (long)m * N);
-    xform(E, tk, w.T, 1, 0, m, m, false, C.stream);
-  }
-  keyswitch_core(C, w, w.T, D2, evk, level);
-  keyswitch_finish(C, w, out->d, half, D0, D0 + half, level, do_rescale);
-  out->level = do_rescale ? level - 1 : level;
-  out->slots = slots;
-  out->scale = scale_after_mult(E, sa, sb, level);
-  out->domain = tk;
+  moddown_conv(E, w.KS + (long)m * N, ks_stride, w.Y, (long)E.k * N, 2, m, C.stream);
+  xform(E, C.transform, w.Y, 2, 0, m, E.k, true, C.stream);
+  ks_combine(E, out, 0, base, 0, w.KS, 0, w.Y, 0, m, 1, 0, C.stream);
+  ks_combine(E, out + half, 0, nullptr, 0, w.KS + ks_stride, 0, w.Y + (long)E.k * N, 0, m, 1, 0, C.stream);
 }
 
 static void hmult_check(const Engine& E, const aoa_ct* a, const aoa_ct* b, const aoa_swk* evk) {
@@ -254,22 +154,38 @@ static void hmult_check(const Engine& E, const aoa_ct* a, const aoa_ct* b, const
   if (E.kl == 0) throw AoaError(AOA_ERR_BAD_PARAM, "key switching needs special primes (kl > 0)");
 }
 
-void hmult(Ctx& C, aoa_ct* out, aoa_ct* a, aoa_ct* b, const aoa_swk* evk, bool do_rescale) {
-  hmult_check(*C.E, a, b, evk);
-  hmult_core(C, get_ws(C), out, a, b, evk, do_rescale);
-}
+static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* const* out, aoa_ct* const* a,
+                        aoa_ct* const* b, const aoa_swk* evk, bool do_rescale, int level);
 
-// Same pipeline on caller-provided scratch of workspace_words(E) words.
+// HMult + relinearisation (ckks_mul_without_rescale, ckks.cpp:273-332),
+// optionally followed by the rescale of ckks_mul (ckks.cpp:334-347), on scratch
+// of workspace_words(E) words: the batched pipeline with one product.  The
+// result is left in the transform domain (the reference leaves coefficients;
+// the residues of every live limb are the same after a domain change).
 void hmult_with_scratch(Ctx& C, aoa_ct* out, aoa_ct* a, aoa_ct* b, const aoa_swk* evk, bool do_rescale,
                         uint64_t* scratch) {
   hmult_check(*C.E, a, b, evk);
-  hmult_core(C, carve(*C.E, scratch), out, a, b, evk, do_rescale);
+  if (evk->domain != C.transform)
+    throw AoaError(AOA_ERR_BAD_PARAM, "the switching key is in another transform domain");
+  // operands to the transform domain, in place (poly_mul does the same, poly_t.cpp:201-220)
+  to_domain(C, a, C.transform, a->level + 1);
+  if (b != a) to_domain(C, b, C.transform, b->level + 1);
+  hmult_group(C, C.stream, scratch, 1, &out, &a, &b, evk, do_rescale, std::min(a->level, b->level));
 }
+
+void hmult(Ctx& C, aoa_ct* out, aoa_ct* a, aoa_ct* b, const aoa_swk* evk, bool do_rescale) {
+  hmult_check(*C.E, a, b, evk);
+  hmult_with_scratch(C, out, a, b, evk, do_rescale, get_scratch(C));
+}
+
+static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* const* out, aoa_ct* const* in,
+                         const long* galois, const aoa_swk* const* keys, int level);
 
 // Galois automorphism X -> X^g followed by the key switch with `key`
 // (ckks_rotate_left/right, ckks.cpp:953-1009; ckks_conjugate, ckks.cpp:1011-1040).
-// The automorphism is applied in the transform domain as a permutation of the
-// evaluation points (the reference permutes coefficients with a sign).
+// On the NTT the automorphism is a permutation of the evaluation points (the
+// reference permutes coefficients with a sign): the batched pipeline with one
+// operation.
 void apply_galois(Ctx& C, aoa_ct* out, aoa_ct* in, long galois, const aoa_swk* key) {
   const Engine& E = *C.E;
   const long N = E.N;
@@ -277,37 +193,29 @@ void apply_galois(Ctx& C, aoa_ct* out, aoa_ct* in, long galois, const aoa_swk* k
   if (E.kl == 0) throw AoaError(AOA_ERR_BAD_PARAM, "key switching needs special primes (kl > 0)");
   const int level = in->level, m = level + 1;
   const long half = (long)E.k * N;
-  Workspace w = get_ws(C);
+  uint64_t* scratch = get_scratch(C);
+  const int tk = C.transform;
+  if (key->domain != tk) throw AoaError(AOA_ERR_BAD_PARAM, "the switching key is in another transform domain");
+  if (tk == AOA_NTT) {
+    to_domain(C, in, AOA_NTT, m);
+    galois_group(C, C.stream, scratch, 1, &out, &in, &galois, &key, level);
+    return;
+  }
+  // Galois maps do not permute the DGT's evaluation points: apply X -> X^g
+  // to the coefficients (as the reference does, aoa-dgt src/tool/encoder.cu:
+  // 338-470) and transform the results.
+  const Workspace w = carve(E, scratch);
   uint64_t* X = w.D + 2 * half;
   const int slots = in->slots;
   const uint64_t scale = in->scale;
-  const int tk = C.transform;
-  if (tk == AOA_DGT) {
-    // Galois maps do not permute the DGT's evaluation points: apply X -> X^g
-    // to the coefficients (as the reference does, aoa-dgt src/tool/encoder.cu:
-    // 338-470) and transform the results.
-    to_domain(C, in, AOA_COEF, m);
-    automorph_coef_op(E, w.R0, in->d, 0, galois, m, 1, C.stream);
-    automorph_coef_op(E, w.T, in->d + half, 0, galois, m, 1, C.stream);
-    copy_limbs(C, X, w.T, (long)m * N);
-    xform(E, tk, X, 1, 0, m, m, true, C.stream);
-    xform(E, tk, w.R0, 1, 0, m, m, true, C.stream);
-  } else {
-    to_domain(C, in, AOA_NTT, m);
-    automorph_ntt_op(E, w.R0, in->d, 0, galois, m, 1, C.stream);
-    automorph_ntt_op(E, X, in->d + half, 0, galois, m, 1, C.stream);
-    if (fused(C, kFuseSource)) {
-      NttIo io;                                // inverse read out of place
-      io.src = X;
-      io.src_poly_stride = m;
-      ntt_batch_io(E, w.T, 1, 0, m, m, false, io, C.stream);
-    } else {
-      copy_limbs(C, w.T, X, (long)m * N);
-      ntt_batch(E, w.T, 1, 0, m, m, false, C.stream);
-    }
-  }
+  to_domain(C, in, AOA_COEF, m);
+  automorph_coef_op(E, w.R0, in->d, 0, galois, m, 1, C.stream);
+  automorph_coef_op(E, w.T, in->d + half, 0, galois, m, 1, C.stream);
+  copy_limbs(C, X, w.T, (long)m * N);
+  xform(E, tk, X, 1, 0, m, m, true, C.stream);
+  xform(E, tk, w.R0, 1, 0, m, m, true, C.stream);
   keyswitch_core(C, w, w.T, X, key, level);
-  keyswitch_finish(C, w, out->d, half, w.R0, nullptr, level, false);
+  keyswitch_finish(C, w, out->d, half, w.R0, level);
   out->level = level;
   out->slots = slots;
   out->scale = scale;
@@ -324,13 +232,9 @@ static size_t batch_words(const Engine& E, int n) {
   return (size_t)E.N * n * (8 * E.k + 3 * std::max(E.kl, 1) + 4);
 }
 
-static void hmult_batch_group(Ctx& C, cudaStream_t st, void*& ws, size_t& ws_bytes, int n, aoa_ct* const* out,
-                              aoa_ct* const* a, aoa_ct* const* b, const aoa_swk* evk, bool do_rescale, int level) {
-  const Engine& E = *C.E;
-  const long N = E.N;
-  const int m = level + 1, k = E.k, kl = E.kl;
-  const long half = (long)k * N, ks = (long)(k + kl) * N;
-  const size_t need = batch_words(E, n) * 8;
+// a stream's batch workspace of at least `words` words
+static uint64_t* batch_ws(cudaStream_t st, void*& ws, size_t& ws_bytes, size_t words) {
+  const size_t need = words * 8;
   if (ws_bytes < need) {
     if (ws) AOA_CUDA(cudaFreeAsync(ws, st));
     ws = nullptr;
@@ -341,7 +245,15 @@ static void hmult_batch_group(Ctx& C, cudaStream_t st, void*& ws, size_t& ws_byt
     }
     ws_bytes = need;
   }
-  uint64_t* p = (uint64_t*)ws;
+  return (uint64_t*)ws;
+}
+
+static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* const* out, aoa_ct* const* a,
+                        aoa_ct* const* b, const aoa_swk* evk, bool do_rescale, int level) {
+  const Engine& E = *C.E;
+  const long N = E.N;
+  const int m = level + 1, k = E.k, kl = E.kl;
+  const long half = (long)k * N, ks = (long)(k + kl) * N;
   uint64_t* D = p;  p += 3L * n * half;
   uint64_t* T = p;  p += (long)n * half;
   uint64_t* UB = p; p += (long)n * kl * N;
@@ -363,12 +275,26 @@ static void hmult_batch_group(Ctx& C, cudaStream_t st, void*& ws, size_t& ws_byt
   // transform with Gaussian-integer products; the fused transform ends are NTT only
   const int tk = C.transform;
   uint64_t* D2 = D + 2L * n * half;
+  const int fuse = tk == AOA_NTT ? E.tune.fuse : 0;
+  OutPtrs outp;
+  for (int z = 0; z < n; z++) {
+    outp.p[z] = out[z]->d;
+    outp.p[n + z] = out[z]->d + half;
+  }
+  // The Q limbs in one last pass over the operands (ks_finish.cu): only d2 is
+  // formed up front.  Not on the DGT, not with the fused transform ends, and
+  // not when one product's output is another's operand (the last pass of the
+  // one may run before the other's has read it).
+  bool late = tk == AOA_NTT && !(fuse & (kFuseKeyProduct | kFuseCombine));
+  for (int x = 0; x < n && late; x++)
+    for (int z = 0; z < n; z++) late = late && (x == z || (out[x] != a[z] && out[x] != b[z]));
   if (tk == AOA_DGT) {
     gi_tensor_batch_op(E, ptr, half, D, n, m, st);
+  } else if (late) {
+    tensor_d2_op(E, ptr, half, D2, n, m, st);
   } else {
     tensor_batch_op(E, ptr, half, D, n, m, st);
   }
-  const int fuse = tk == AOA_NTT ? E.tune.fuse : 0;
   if (fuse & kFuseSource) {
     NttIo io;                                  // inverse of d2 read in place of a copy
     io.src = D2;
@@ -394,15 +320,22 @@ static void hmult_batch_group(Ctx& C, cudaStream_t st, void*& ws, size_t& ws_byt
     keyswitch_mul_batch_op(E, D2, half, nullptr, 0, evk->d, KS, ks, n, m, st, 0);
   } else {
     ntt_batch(E, UB, n, k, kl, kl, true, st);
-    keyswitch_mul_batch_op(E, D2, half, UB, (long)kl * N, evk->d, KS, ks, n, m, st);
+    if (late) keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, evk->d, KS + (long)m * N, ks, n, 0, st);
+    else keyswitch_mul_batch_op(E, D2, half, UB, (long)kl * N, evk->d, KS, ks, n, m, st);
   }
   xform(E, tk, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
-  OutPtrs outp;
-  for (int z = 0; z < n; z++) {
-    outp.p[z] = out[z]->d;
-    outp.p[n + z] = out[z]->d + half;
-  }
-  if (do_rescale) {
+  if (late) {
+    if (do_rescale) {
+      hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
+      ntt_batch(E, U, 2 * n, level, 1, 1, false, st);
+      rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st);
+    } else {
+      moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+    }
+    const int nl = do_rescale ? level : m;
+    ntt_batch(E, Y, 2 * n, 0, nl, k, true, st);
+    hmult_finish_op(E, ptr, half, D2, evk->d, Y, outp, n, nl, do_rescale ? level : 0, st);
+  } else if (do_rescale) {
     ks_combine(E, U, N, D + (long)level * N, half, KS + (long)level * N, ks, nullptr, 0, 1, 2 * n, 0, st, level);
     xform(E, tk, U, 2 * n, level, 1, 1, false, st);
     rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st);
@@ -540,7 +473,7 @@ void hmult_batch(Ctx& C, int n, aoa_ct* const* out, aoa_ct* const* a, aoa_ct* co
   run_grouped(C, n, out, a, b, [&](int z) { return std::min(a[z]->level, b[z]->level); },
               [&](cudaStream_t st, void*& ws, size_t& wb, int g, aoa_ct* const* go, aoa_ct* const* ga,
                   aoa_ct* const* gb, int level, const int*) {
-                hmult_batch_group(C, st, ws, wb, g, go, ga, gb, evk, do_rescale, level);
+                hmult_group(C, st, batch_ws(st, ws, wb, batch_words(E, g)), g, go, ga, gb, evk, do_rescale, level);
               });
 }
 
@@ -553,24 +486,12 @@ static size_t galois_words(const Engine& E, int n) {
   return (size_t)E.N * n * (3 * E.k + E.kl + 2 * (E.k + E.kl) + 2 * E.k);
 }
 
-static void galois_batch_group(Ctx& C, cudaStream_t st, void*& ws, size_t& ws_bytes, int n, aoa_ct* const* out,
-                               aoa_ct* const* in, const long* galois, const aoa_swk* const* keys, int level) {
+static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* const* out, aoa_ct* const* in,
+                         const long* galois, const aoa_swk* const* keys, int level) {
   const Engine& E = *C.E;
   const long N = E.N;
   const int m = level + 1, k = E.k, kl = E.kl;
   const long half = (long)k * N, ks = (long)(k + kl) * N;
-  const size_t need = galois_words(E, n) * 8;
-  if (ws_bytes < need) {
-    if (ws) AOA_CUDA(cudaFreeAsync(ws, st));
-    ws = nullptr;
-    ws_bytes = 0;
-    if (cudaMallocAsync(&ws, need, st) != cudaSuccess) {
-      cudaGetLastError();
-      throw AoaError(AOA_ERR_OOM, "batch workspace allocation failed");
-    }
-    ws_bytes = need;
-  }
-  uint64_t* p = (uint64_t*)ws;
   uint64_t* R = p;  p += 2L * n * half;
   uint64_t* T = p;  p += (long)n * half;
   uint64_t* UB = p; p += (long)n * kl * N;
@@ -591,6 +512,21 @@ static void galois_batch_group(Ctx& C, cudaStream_t st, void*& ws, size_t& ws_by
     gl.g[z] = galois[z];
     one_key = one_key && keys[z] == keys[0];
   }
+  KeyPtrs kp;
+  for (int z = 0; z < n; z++) kp.k[z] = keys[z]->d;
+  OutPtrs outp;
+  for (int z = 0; z < n; z++) {
+    outp.p[z] = out[z]->d;
+    outp.p[n + z] = out[z]->d + half;
+  }
+  auto done = [&] {
+    for (int z = 0; z < n; z++) {
+      out[z]->level = level;
+      out[z]->slots = slots[z];
+      out[z]->scale = scale[z];
+      out[z]->domain = AOA_NTT;
+    }
+  };
   automorph_ntt_batch_op(E, ptr, half, R, n, gl, m, st);
   NttIo io;                                      // inverse of the permuted c1, out of place
   io.src = X;
@@ -598,28 +534,16 @@ static void galois_batch_group(Ctx& C, cudaStream_t st, void*& ws, size_t& ws_by
   ntt_batch_io(E, T, n, 0, m, k, false, io, st);
   modup(E, T, half, UB, (long)kl * N, n, level, st);
   ntt_batch(E, UB, n, k, kl, kl, true, st);
-  if (one_key) {                                 // each key word read once for the group
-    keyswitch_mul_batch_op(E, X, half, UB, (long)kl * N, keys[0]->d, KS, ks, n, m, st);
-  } else {
-    KeyPtrs kp;
-    for (int z = 0; z < n; z++) kp.k[z] = keys[z]->d;
-    keyswitch_mul_keys_op(E, X, half, UB, (long)kl * N, kp, KS, ks, n, m, st);
-  }
+  // special limbs' key products; the Q limbs' are formed in the last pass
+  if (one_key)                                   // each key word read once for the group
+    keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, keys[0]->d, KS + (long)m * N, ks, n, 0, st);
+  else
+    keyswitch_mul_keys_op(E, nullptr, 0, UB, (long)kl * N, kp, KS + (long)m * N, ks, n, 0, st);
   ntt_batch(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
   moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
   ntt_batch(E, Y, 2 * n, 0, m, k, true, st);
-  OutPtrs outp;
-  for (int z = 0; z < n; z++) {
-    outp.p[z] = out[z]->d;
-    outp.p[n + z] = out[z]->d + half;
-  }
-  ks_combine_ptr(E, outp, R, half, KS, ks, Y, half, m, 2 * n, 0, st, n);   // c0 base for poly 0 only
-  for (int z = 0; z < n; z++) {
-    out[z]->level = level;
-    out[z]->slots = slots[z];
-    out[z]->scale = scale[z];
-    out[z]->domain = AOA_NTT;
-  }
+  galois_finish_op(E, R, half, kp, one_key, Y, outp, n, m, st);
+  done();
 }
 
 // n automorphisms, op z by galois[z] with keys[z]: grouped by level only, so
@@ -649,7 +573,7 @@ void galois_batch(Ctx& C, int n, aoa_ct* const* out, aoa_ct* const* in, const lo
                   gg[t] = galois[ids[t]];
                   kk[t] = keys[ids[t]];
                 }
-                galois_batch_group(C, st, ws, wb, g, go, ga, gg.data(), kk.data(), level);
+                galois_group(C, st, batch_ws(st, ws, wb, galois_words(E, g)), g, go, ga, gg.data(), kk.data(), level);
               });
 }
 
