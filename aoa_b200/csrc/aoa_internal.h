@@ -60,6 +60,7 @@ struct Tune {
   double ntt_waves = 1.0;             // transform CTAs per pass, in resident waves
   double ntt_waves_large = 8.0;       // the same for launches of at least kLargeItems limbs
   bool conv_tensor_cores = true;      // basis conversion on the int8 tensor cores where it applies
+  bool ntt_shape_set = false;         // a caller chose a shape: no whole-limb kernels
   int ntt_split = 0;                  // log2(C) - floor(log2(N) / 2) of the R x C transform split
   // the same for the DGT's cyclic limb transforms (N/2 points): at N = 2^16
   // the 2^15-point transforms ran 2-3% faster with 256-point rows than with
@@ -293,6 +294,29 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
                       long poly_stride, bool forward, cudaStream_t st, const NttIo* io = nullptr);
 void ntt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int nlimbs,
                long poly_stride, bool forward, cudaStream_t st);
+
+// ntt_limb.cu: whole-limb transforms of N = 2^10 .. 2^14 and the ends of HMult and
+// the automorphisms fused with them.  limb_serves: whether a call of `items`
+// limb transforms takes them.
+void limb_init(const Engine& E);
+bool limb_serves(const Engine& E, int log_n, long items);
+void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
+                    long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, cudaStream_t st);
+// D2 + z half = a1 b1 and T + z half = its inverse transform, op z
+void limb_tensor_inv(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, uint64_t* T, int n, int nlimbs,
+                     cudaStream_t st);
+// R = permuted [c0 | c1] of every op, T = the inverse transform of the permuted c1
+void limb_galois_inv(const Engine& E, const CtPtrs& ptr, const GaloisList& g, long half, uint64_t* R, uint64_t* T,
+                     int n, int nlimbs, cudaStream_t st);
+// special limbs: KS + (part n + z) ks_stride = inverse(forward(UB of op z) key part); with ptr also
+// U + (part n + z) N = inverse of the top limb of d + d2 key B^-1
+void limb_key(const Engine& E, const uint64_t* UB, uint64_t* KS, long ks_stride, const KeyPtrs& keys, int n,
+              const CtPtrs* ptr, long half, const uint64_t* D2, uint64_t* U, int level, cudaStream_t st);
+// forward transform of the corrections Y and the Q limbs out of it
+void limb_finish(const Engine& E, uint64_t* Y, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+                 const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
+void limb_galois_finish(const Engine& E, uint64_t* Y, const uint64_t* R, long half, const KeyPtrs& keys,
+                        const OutPtrs& outp, int n, int nlimbs, cudaStream_t st);
 
 // rns.cu
 void rns_init(Engine& E);

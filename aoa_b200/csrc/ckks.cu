@@ -288,6 +288,35 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
   bool late = tk == AOA_NTT && !(fuse & (kFuseKeyProduct | kFuseCombine));
   for (int x = 0; x < n && late; x++)
     for (int z = 0; z < n; z++) late = late && (x == z || (out[x] != a[z] && out[x] != b[z]));
+  // small rings: five launches, the transforms as whole-limb clusters with the
+  // work around them inside (ntt_limb.cu)
+  const bool whole = late && fuse == kFuseSource && limb_serves(E, E.log_n, 2L * n * (kl + 1)) &&
+                     limb_serves(E, E.log_n, 2L * n * m);
+  if (whole) {
+    limb_tensor_inv(E, ptr, half, D2, T, n, m, st);
+    modup(E, T, half, UB, (long)kl * N, n, level, st);
+    KeyPtrs kp;
+    for (int z = 0; z < n; z++) kp.k[z] = evk->d;
+    limb_key(E, UB, KS + (long)m * N, ks, kp, n, do_rescale ? &ptr : nullptr, half, D2, U, level, st);
+    if (do_rescale) rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st);
+    else moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+    const int nl = do_rescale ? level : m, rl = do_rescale ? level : 0;
+    bool in_place = false;                       // the two polys' clusters run apart: an operand must outlive both
+    for (int z = 0; z < n; z++) in_place = in_place || out[z] == a[z] || out[z] == b[z];
+    if (in_place) {
+      ntt_batch(E, Y, 2 * n, 0, nl, k, true, st);
+      hmult_finish_op(E, ptr, half, D2, evk->d, Y, outp, n, nl, rl, st);
+    } else {
+      limb_finish(E, Y, ptr, half, D2, evk->d, outp, n, nl, rl, st);
+    }
+    for (int z = 0; z < n; z++) {
+      out[z]->level = do_rescale ? level - 1 : level;
+      out[z]->slots = slots[z];
+      out[z]->scale = scale_after_mult(E, sa[z], sb[z], level);
+      out[z]->domain = tk;
+    }
+    return;
+  }
   if (tk == AOA_DGT) {
     gi_tensor_batch_op(E, ptr, half, D, n, m, st);
   } else if (late) {
@@ -527,6 +556,16 @@ static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* co
       out[z]->domain = AOA_NTT;
     }
   };
+  if (E.tune.fuse == kFuseSource && limb_serves(E, E.log_n, 2L * n * kl) && limb_serves(E, E.log_n, 2L * n * m)) {
+    // small rings: whole-limb clusters (as hmult_group)
+    limb_galois_inv(E, ptr, gl, half, R, T, n, m, st);
+    modup(E, T, half, UB, (long)kl * N, n, level, st);
+    limb_key(E, UB, KS + (long)m * N, ks, kp, n, nullptr, 0, nullptr, nullptr, level, st);
+    moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+    limb_galois_finish(E, Y, R, half, kp, outp, n, m, st);
+    done();
+    return;
+  }
   automorph_ntt_batch_op(E, ptr, half, R, n, gl, m, st);
   NttIo io;                                      // inverse of the permuted c1, out of place
   io.src = X;

@@ -343,6 +343,7 @@ int aoa_engine_tune(aoa_engine* h, const char* knob, double value) {
   else if (k == "spin_limit" && value >= 0 && value <= (1 << 30) && value == (int)value)
     h->e.tune.spin_limit = (int)value;
   else return fail(AOA_ERR_BAD_PARAM, "unknown knob or value out of range: " + k);
+  if (k.rfind("ntt_", 0) == 0 || k == "dgt_split") h->e.tune.ntt_shape_set = true;
   return AOA_OK;
 }
 

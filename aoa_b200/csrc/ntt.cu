@@ -19,6 +19,7 @@ void ntt_init(Engine& E) {
   allow_kind<kButterflyLazy>();
   allow_kind<kButterflyLazyQ1>();
   allow_wo_kernels();
+  limb_init(E);
   int sms = 0;
   AOA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E.device));
   E.num_sms = sms;
@@ -100,6 +101,12 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
   if (npolys <= 0 || nlimbs <= 0) return;
   if (first_prime < 0 || first_prime + ((nlimbs - 1) >> T.prime_shift) >= E.nprimes)
     throw AoaError(AOA_ERR_BAD_PARAM, "ntt: prime range out of bounds");
+  if (limb_serves(E, T.log_n, (long)npolys * nlimbs) && (!io || io->epi.mode == kEpiStore)) {
+    check_alignment(data, io);
+    limb_transform(E, T, data, npolys, first_prime, nlimbs, poly_stride, forward, io ? io->src : nullptr,
+                   io ? io->src_poly_stride : 0, st);
+    return;
+  }
   if (T.prime_kind && T.log_n >= 10) {
     // Primes of different butterfly kinds (the reference's prime sets put a
     // 63-bit q0 before its 45..55-bit buckets): the limbs run in maximal runs

@@ -110,7 +110,9 @@ int aoa_engine_destroy(aoa_engine* e);
  * "spin_limit" (polls of the kernels' bounded mbarrier waits before they
  * give up and report AOA_ERR_TIMEOUT at the next aoa_ctx_sync, 0..2^30;
  * default 2^20; the drain of copies and MMAs in flight after an expired
- * wait always uses the default bound).                                     */
+ * wait always uses the default bound).  Rings up to 2^14 run small calls as
+ * one whole-limb kernel per transform, which has no shape to choose: setting
+ * any "ntt_*" knob or "dgt_split" keeps the engine on the two-pass kernels. */
 int aoa_engine_tune(aoa_engine* e, const char* knob, double value);
 /* current value of a knob (names as for aoa_engine_tune) */
 int aoa_engine_tune_get(const aoa_engine* e, const char* knob, double* value);
