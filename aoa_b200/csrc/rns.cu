@@ -164,6 +164,7 @@ basis_convert(ConvArgs a, int j_first, int j_end) {
 constexpr int kTcRowsLog = 7;
 constexpr int kTcRows = 1 << kTcRowsLog;
 constexpr int kTcThreads = 512;
+constexpr int kTcPerSm = 2;        // CTAs per SM: 97 KiB of shared memory, 256 tensor-memory columns each
 constexpr int kTcN = 256;
 constexpr size_t kTcA = 16 * kTcRows * 16;
 constexpr size_t kTcB = 16 * kTcN * 16;
@@ -283,15 +284,21 @@ __device__ __forceinline__ uint64_t tc_cross(uint64_t x, uint64_t p, const TcOut
   return tc_shoup<Q1>(x, 1, c.one_sh, c.q);
 }
 
+// Two CTAs of 16 warps share an SM (64 registers a thread): alone, a CTA spent
+// 1440 of the 6400 cycles of a ModUp tile waiting for its MMAs and 350 at its
+// barriers, and its four warps per scheduler issued half the time in the rest.
+// Measured against one CTA per SM: 12 rotations at 2^16 2234 -> 2156 us, 48 HMults
+// 9765 -> 9579 us.
 // Persistent: CTA b handles tiles b, b + grid, ...  Per tile: the inputs (loaded
 // into registers during the previous tile's MMA and epilogue) are scaled and
 // written to A, one thread issues the MMAs and commits them to an mbarrier,
 // and all 16 warps read tensor memory: warp w owns lanes 32 (w % 4) .. + 31
 // (tile rows) and every fourth output starting at w / 4.
-constexpr int kTcPairs = 32 / 2 / (kTcThreads / kTcRows);   // input pairs per thread (nin <= 32)
+constexpr int kTcGroups = kTcThreads / kTcRows;             // threads per tile row
+constexpr int kTcPairs = (16 + kTcGroups - 1) / kTcGroups;   // input pairs per thread (nin <= 32)
 
 template <int MODE, bool Q1>
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kTcThreads, kTcPerSm)
 basis_convert_tc(ConvArgs a, int j_first, int j_end) {
   extern __shared__ __align__(1024) uint8_t tcs[];
   __shared__ __align__(8) uint64_t mbar[2];                // [0] image loaded, [1] MMA done
@@ -415,7 +422,7 @@ basis_convert_tc(ConvArgs a, int j_first, int j_end) {
       // the rescale modes read the table with B^-1 folded in: sums are conv * B^-1
       const uint64_t sl = (l & 1) ? tc_combine<Q1>(v + 8, cpl, Pl) : tc_combine<Q1>(v, cpl, Pl);
       const uint64_t cl = sub_mod(dv, sl, cpl.q);
-      const int per = (((l + 3) / 4) + 1) & ~1;
+      const int per = (((l + kTcGroups - 1) / kTcGroups) + 1) & ~1;
       const int jb = par * per, je = min(l, jb + per);
       for (int j = jb; j < je; j += 2) {
         tc_ld16(t_lane + j * 8, v);
@@ -431,7 +438,7 @@ basis_convert_tc(ConvArgs a, int j_first, int j_end) {
       }
     } else {
       const int nout = j_end - j_first;
-      const int per = (((nout + 3) / 4) + 1) & ~1;
+      const int per = (((nout + kTcGroups - 1) / kTcGroups) + 1) & ~1;
       const int jb = j_first + par * per, je = min(j_end, jb + per);
       for (int jj = jb & ~1; jj < je; jj += 2) {
         tc_ld16(t_lane + jj * 8, v);
@@ -480,7 +487,7 @@ static void run_convert(const Engine& E, const ConvArgs& a, int npolys, int j_be
     t.spin = E.tune.spin_limit;
     t.npolys = npolys;
     const long tiles = (N / kTcRows) * npolys;
-    const unsigned grid_tc = (unsigned)std::min<long>(tiles, E.num_sms);
+    const unsigned grid_tc = (unsigned)std::min<long>(tiles, (long)kTcPerSm * E.num_sms);
     bool q1 = true;                               // every input and output prime q = 1 mod 2^32 below 2^60
     for (int i = 0; i < a.nin; i++) q1 = q1 && E.prime_kind[a.in_prime0 + i] == kButterflyLazyQ1;
     for (int j = 0; j < j_end; j++) q1 = q1 && E.prime_kind[a.out_prime0 + j] == kButterflyLazyQ1;
