@@ -297,9 +297,9 @@ void ntt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int
 
 // ntt_limb.cu: whole-limb transforms of N = 2^10 .. 2^14 and the ends of HMult and
 // the automorphisms fused with them.  limb_serves: whether a call of `items`
-// limb transforms takes them.
+// limb transforms (plain, or the fused ends of a key switch) takes them.
 void limb_init(const Engine& E);
-bool limb_serves(const Engine& E, int log_n, long items);
+bool limb_serves(const Engine& E, int log_n, long items, bool fused);
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
                     long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, cudaStream_t st);
 // D2 + z half = a1 b1 and T + z half = its inverse transform, op z

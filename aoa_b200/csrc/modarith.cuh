@@ -125,11 +125,11 @@ __device__ __forceinline__ uint64_t shoup_lazy_mad3_q1(uint64_t y, uint64_t w, u
       "addc.u32 t1, t1, 0;\n\t"
       "mul.wide.u32 R, y0, w0;\n\t"
       "mov.b64 {r0, r1}, R;\n\t"
-      "sub.cc.u32 r0, r0, t0;\n\t"
-      "subc.u32 r1, r1, t1;\n\t"
       "mad.lo.u32 r1, y0, w1, r1;\n\t"
       "mad.lo.u32 r1, y1, w0, r1;\n\t"
       "mad.lo.u32 r1, t0, %4, r1;\n\t"
+      "sub.cc.u32 r0, r0, t0;\n\t"
+      "subc.u32 r1, r1, t1;\n\t"
       "mov.b64 %0, {r0, r1};\n\t"
       "}"
       : "=l"(r)

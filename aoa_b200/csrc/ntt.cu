@@ -101,7 +101,7 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
   if (npolys <= 0 || nlimbs <= 0) return;
   if (first_prime < 0 || first_prime + ((nlimbs - 1) >> T.prime_shift) >= E.nprimes)
     throw AoaError(AOA_ERR_BAD_PARAM, "ntt: prime range out of bounds");
-  if (limb_serves(E, T.log_n, (long)npolys * nlimbs) && (!io || io->epi.mode == kEpiStore)) {
+  if (limb_serves(E, T.log_n, (long)npolys * nlimbs, false) && (!io || io->epi.mode == kEpiStore)) {
     check_alignment(data, io);
     limb_transform(E, T, data, npolys, first_prime, nlimbs, poly_stride, forward, io ? io->src : nullptr,
                    io ? io->src_poly_stride : 0, st);

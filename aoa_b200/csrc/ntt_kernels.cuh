@@ -860,6 +860,10 @@ ntt_rows(NttBatch b, const __grid_constant__ NttEpi epi) {
 
 // CTAs per tile column: about one resident wave of CTAs (blocks_per_sm per SM)
 static inline int ctas_per_tile(const Engine& E, int tiles, int items, int blocks_per_sm) {
+  // Calls of up to two and a half waves run one tile per CTA: with one wave of
+  // CTAs some of them hold two tiles and some three (31 limbs in 27 groups at
+  // 2^16: two for 4 groups, one for 23), and the pass ends with the longest.
+  if ((double)items * tiles <= 2.5 * E.num_sms * blocks_per_sm) return items;
   // large launches balance better with more, shorter-lived CTAs (the hardware
   // hands later waves to the SMs that finish first); small ones pay per CTA
   const double waves = items >= kLargeItems ? E.tune.ntt_waves_large : E.tune.ntt_waves;

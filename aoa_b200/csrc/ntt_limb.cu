@@ -559,10 +559,12 @@ void limb_init(const Engine&) {
 // HMult with 12 limbs (28 key-product limbs) 55.3 -> 34.9 at 2^12, 97.8 -> 63.6
 // at 2^14, 124.5 -> 121.7 at 2^15; four of them (112) 118.8 -> 113.4 at 2^13,
 // 171.6 -> 207.9 at 2^14; rotation with 20 limbs (42) 103.1 -> 99.6 at 2^14,
-// 148.6 -> 189.5 at 2^15.
-bool limb_serves(const Engine& E, int log_n, long items) {
-  constexpr long kMost[] = {1024, 1024, 320, 112, 56, 20};   // log_n = 10 .. 15
-  return !E.tune.ntt_shape_set && log_n >= 10 && log_n <= 15 && items <= kMost[log_n - 10];
+// 148.6 -> 189.5 at 2^15.  A plain transform (two launches saved to one) and the
+// fused ends of a key switch (`fused`: its 2 n (kl + 1) key-product limbs) have
+// a line each.
+bool limb_serves(const Engine& E, int log_n, long items, bool fused) {
+  constexpr long kMost[2][6] = {{1024, 1024, 448, 128, 64, 8}, {1024, 1024, 320, 112, 56, 20}};   // log_n = 10 .. 15
+  return !E.tune.ntt_shape_set && log_n >= 10 && log_n <= 15 && items <= kMost[fused][log_n - 10];
 }
 
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
