@@ -316,7 +316,7 @@ void limb_key(const Engine& E, const uint64_t* UB, uint64_t* KS, long ks_stride,
 void limb_finish(const Engine& E, uint64_t* Y, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
                  const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
 void limb_galois_finish(const Engine& E, uint64_t* Y, const uint64_t* R, long half, const KeyPtrs& keys,
-                        const OutPtrs& outp, int n, int nlimbs, cudaStream_t st);
+                        const OutPtrs& outp, int n, int nlimbs, bool add, cudaStream_t st);
 
 // rns.cu
 void rns_init(Engine& E);
@@ -378,7 +378,7 @@ void hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t*
 void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
 void galois_finish_op(const Engine& E, const uint64_t* R, long half, const KeyPtrs& keys, bool one_key,
-                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, cudaStream_t st);
+                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, bool add, cudaStream_t st);
 void automorph_ntt_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* out, int n,
                             const GaloisList& galois, int nlimbs, cudaStream_t st);
 // key products with a key per op (keys.k[z], [b | a] over all primes)

@@ -179,14 +179,15 @@ void hmult(Ctx& C, aoa_ct* out, aoa_ct* a, aoa_ct* b, const aoa_swk* evk, bool d
 }
 
 static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* const* out, aoa_ct* const* in,
-                         const long* galois, const aoa_swk* const* keys, int level);
+                         const long* galois, const aoa_swk* const* keys, int level, bool add = false);
 
 // Galois automorphism X -> X^g followed by the key switch with `key`
 // (ckks_rotate_left/right, ckks.cpp:953-1009; ckks_conjugate, ckks.cpp:1011-1040).
 // On the NTT the automorphism is a permutation of the evaluation points (the
 // reference permutes coefficients with a sign): the batched pipeline with one
 // operation.
-void apply_galois(Ctx& C, aoa_ct* out, aoa_ct* in, long galois, const aoa_swk* key) {
+// add_to_out: out, which is in, becomes in + its image (NTT contexts).
+void apply_galois(Ctx& C, aoa_ct* out, aoa_ct* in, long galois, const aoa_swk* key, bool add_to_out = false) {
   const Engine& E = *C.E;
   const long N = E.N;
   if (!key || !key->d) throw AoaError(AOA_ERR_NO_KEY, "missing switching key for this automorphism");
@@ -198,7 +199,7 @@ void apply_galois(Ctx& C, aoa_ct* out, aoa_ct* in, long galois, const aoa_swk* k
   if (key->domain != tk) throw AoaError(AOA_ERR_BAD_PARAM, "the switching key is in another transform domain");
   if (tk == AOA_NTT) {
     to_domain(C, in, AOA_NTT, m);
-    galois_group(C, C.stream, scratch, 1, &out, &in, &galois, &key, level);
+    galois_group(C, C.stream, scratch, 1, &out, &in, &galois, &key, level, add_to_out);
     return;
   }
   // Galois maps do not permute the DGT's evaluation points: apply X -> X^g
@@ -516,7 +517,7 @@ static size_t galois_words(const Engine& E, int n) {
 }
 
 static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* const* out, aoa_ct* const* in,
-                         const long* galois, const aoa_swk* const* keys, int level) {
+                         const long* galois, const aoa_swk* const* keys, int level, bool add) {
   const Engine& E = *C.E;
   const long N = E.N;
   const int m = level + 1, k = E.k, kl = E.kl;
@@ -563,7 +564,7 @@ static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* co
     modup(E, T, half, UB, (long)kl * N, n, level, st);
     limb_key(E, UB, KS + (long)m * N, ks, kp, n, nullptr, 0, nullptr, nullptr, level, st);
     moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
-    limb_galois_finish(E, Y, R, half, kp, outp, n, m, st);
+    limb_galois_finish(E, Y, R, half, kp, outp, n, m, add, st);
     done();
     return;
   }
@@ -582,7 +583,7 @@ static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* co
   ntt_batch(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
   moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
   ntt_batch(E, Y, 2 * n, 0, m, k, true, st);
-  galois_finish_op(E, R, half, kp, one_key, Y, outp, n, m, st);
+  galois_finish_op(E, R, half, kp, one_key, Y, outp, n, m, add, st);
   done();
 }
 

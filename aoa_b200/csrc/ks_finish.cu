@@ -98,11 +98,13 @@ __global__ void __launch_bounds__(kThreads) hmult_finish(const __grid_constant__
 
 // out0 = r0 + (x kb - y0) B^-1, out1 = (x ka - y1) B^-1 with r0 = R, x = R + n
 // half the permuted polys of op z at op stride half; key of op z keys.k[z].
+// add: the outputs' words are added to (a rotate-and-sum step).
 template <bool ONE_KEY>
 __global__ void __launch_bounds__(kThreads) galois_finish(const uint64_t* R, long half,
                                                           const __grid_constant__ KeyPtrs keys, long key_half,
                                                           const uint64_t* Y, const __grid_constant__ OutPtrs outp,
-                                                          int n, const ShoupW* binv, const PrimeConst* pc, int log_n) {
+                                                          int n, bool add, const ShoupW* binv, const PrimeConst* pc,
+                                                          int log_n) {
   pdl_begin();
   const int i = blockIdx.y;
   const PrimeConst P = pc[i];
@@ -121,10 +123,20 @@ __global__ void __launch_bounds__(kThreads) galois_finish(const uint64_t* R, lon
     }
     const ulonglong2 r0 = ld2(R + (long)z * half + off), x = ld2(R + (long)(n + z) * half + off);
     const ulonglong2 y0 = ld2(Y + (long)z * half + off), y1 = ld2(Y + (long)(n + z) * half + off);
-    st2(outp.p[z] + off, add_mod(r0.x, shoup(sub_mod(mul_mod(x.x, kb.x, P), y0.x, q), bi, q), q),
-        add_mod(r0.y, shoup(sub_mod(mul_mod(x.y, kb.y, P), y0.y, q), bi, q), q));
-    st2(outp.p[n + z] + off, shoup(sub_mod(mul_mod(x.x, ka.x, P), y1.x, q), bi, q),
-        shoup(sub_mod(mul_mod(x.y, ka.y, P), y1.y, q), bi, q));
+    ulonglong2 c0, c1;
+    c0.x = add_mod(r0.x, shoup(sub_mod(mul_mod(x.x, kb.x, P), y0.x, q), bi, q), q);
+    c0.y = add_mod(r0.y, shoup(sub_mod(mul_mod(x.y, kb.y, P), y0.y, q), bi, q), q);
+    c1.x = shoup(sub_mod(mul_mod(x.x, ka.x, P), y1.x, q), bi, q);
+    c1.y = shoup(sub_mod(mul_mod(x.y, ka.y, P), y1.y, q), bi, q);
+    if (add) {
+      const ulonglong2 o0 = ld2(outp.p[z] + off), o1 = ld2(outp.p[n + z] + off);
+      c0.x = add_mod(c0.x, o0.x, q);
+      c0.y = add_mod(c0.y, o0.y, q);
+      c1.x = add_mod(c1.x, o1.x, q);
+      c1.y = add_mod(c1.y, o1.y, q);
+    }
+    st2(outp.p[z] + off, c0.x, c0.y);
+    st2(outp.p[n + z] + off, c1.x, c1.y);
   }
 }
 
@@ -158,11 +170,11 @@ void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64
 }
 
 void galois_finish_op(const Engine& E, const uint64_t* R, long half, const KeyPtrs& keys, bool one_key,
-                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, cudaStream_t st) {
+                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, bool add, cudaStream_t st) {
   const long blocks = E.N / (2 * kThreads) * nlimbs;
   const dim3 grid(E.N / (2 * kThreads), nlimbs, op_blocks(E, blocks, n));
   launch_pdl(one_key ? galois_finish<true> : galois_finish<false>, grid, kThreads, 0, st, R, half, keys,
-             (long)E.nprimes * E.N, Y, outp, n, E.rns.moddown_binv, E.d_pc, E.log_n);
+             (long)E.nprimes * E.N, Y, outp, n, add, E.rns.moddown_binv, E.d_pc, E.log_n);
 }
 
 }  // namespace aoa

@@ -99,6 +99,7 @@ struct GaloisFinishEnds {
   long key_half;
   OutPtrs outp;
   int n;
+  bool add;                // add to the outputs' words
   const ShoupW* binv;
 };
 template <int MODE> struct EndsOf { using T = NoEnds; };
@@ -369,7 +370,8 @@ __device__ __forceinline__ void limb_run(const LimbArgs& a, const typename EndsO
     for (int i = tid; i < L::M; i += L::P) {
       const uint64_t y = Bf<KIND>::fwd_out(lds64(word(i)), q);
       const uint64_t d = shoup(sub_mod(mul_mod(X[i], key[i], P), y, q), bi, q);
-      out[i] = second ? d : add_mod(R0[i], d, q);
+      const uint64_t c = second ? d : add_mod(R0[i], d, q);
+      out[i] = e.add ? add_mod(out[i], c, q) : c;
     }
   } else {
     if constexpr (MODE == kLimbInv) {
@@ -657,7 +659,7 @@ void limb_finish(const Engine& E, uint64_t* Y, const CtPtrs& ptr, long half, con
 }
 
 void limb_galois_finish(const Engine& E, uint64_t* Y, const uint64_t* R, long half, const KeyPtrs& keys,
-                        const OutPtrs& outp, int n, int nlimbs, cudaStream_t st) {
+                        const OutPtrs& outp, int n, int nlimbs, bool add, cudaStream_t st) {
   LimbArgs a = limb_args(E);
   a.data = Y;
   a.poly_stride = half >> E.log_n;
@@ -669,6 +671,7 @@ void limb_galois_finish(const Engine& E, uint64_t* Y, const uint64_t* R, long ha
   e.key_half = (long)E.nprimes * E.N;
   e.outp = outp;
   e.n = n;
+  e.add = add;
   e.binv = E.rns.moddown_binv;
   limb_dispatch<kLimbGaloisFinish>(E.log_n, a, e, nlimbs, st);
 }

@@ -11,7 +11,7 @@ using namespace aoa;
 
 namespace aoa {
 void ct_to_domain(Ctx& C, aoa_ct* ct, int domain, int nlimbs);
-void apply_galois(Ctx& C, aoa_ct* out, aoa_ct* in, long galois, const aoa_swk* key);
+void apply_galois(Ctx& C, aoa_ct* out, aoa_ct* in, long galois, const aoa_swk* key, bool add_to_out = false);
 }  // namespace aoa
 
 namespace {
@@ -182,8 +182,10 @@ int aoa_sumslots(aoa_ctx* c, aoa_ct* out, aoa_ct* in, const aoa_swk* const* rtks
       AOA_CUDA(cudaMemcpyAsync(out->d, in->d, bytes, cudaMemcpyDeviceToDevice, C.stream));
       copy_meta(out, in);
     }
+    // each step adds the rotation to `out` in its last pass on the NTT; the
+    // DGT's automorphisms pass through coefficients and a temporary
     aoa_ct tmp;
-    if (cudaMallocAsync(&tmp.d, bytes, C.stream) != cudaSuccess) {
+    if (C.transform == AOA_DGT && cudaMallocAsync(&tmp.d, bytes, C.stream) != cudaSuccess) {
       cudaGetLastError();
       throw AoaError(AOA_ERR_OOM, "sumslots buffer allocation failed");
     }
@@ -197,16 +199,20 @@ int aoa_sumslots(aoa_ctx* c, aoa_ct* out, aoa_ct* in, const aoa_swk* const* rtks
           while (e) { if (e & 1) r = r * b % M; b = b * b % M; e >>= 1; }
           return r;
         }();
+        if (C.transform == AOA_NTT) {
+          apply_galois(C, out, out, g, rtks[j], true);
+          continue;
+        }
         apply_galois(C, &tmp, out, g, rtks[j]);
         ct_to_domain(C, out, tmp.domain, out->level + 1);
         ew_binary_op(E, out->d, (long)E.k * E.N, out->d, (long)E.k * E.N, tmp.d, (long)E.k * E.N, 0, 0,
                      out->level + 1, 2, C.stream);
       }
     } catch (...) {
-      cudaFreeAsync(tmp.d, C.stream);
+      if (tmp.d) cudaFreeAsync(tmp.d, C.stream);
       throw;
     }
-    AOA_CUDA(cudaFreeAsync(tmp.d, C.stream));
+    if (tmp.d) AOA_CUDA(cudaFreeAsync(tmp.d, C.stream));
   });
 }
 
