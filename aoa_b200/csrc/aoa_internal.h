@@ -376,6 +376,13 @@ void tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, i
 void hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key, uint64_t* U,
                   int n, int level, cudaStream_t st);
 void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+// the same with Gaussian-integer products (DGT domain, planar limbs)
+void gi_tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, int n, int nlimbs, cudaStream_t st);
+void gi_hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+                     uint64_t* U, int n, int level, cudaStream_t st);
+void gi_hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+                        const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level,
+                        cudaStream_t st);
                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
 void galois_finish_op(const Engine& E, const uint64_t* R, long half, const KeyPtrs& keys, bool one_key,
                       const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, bool add, cudaStream_t st);

@@ -283,10 +283,10 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
     outp.p[n + z] = out[z]->d + half;
   }
   // The Q limbs in one last pass over the operands (ks_finish.cu): only d2 is
-  // formed up front.  Not on the DGT, not with the fused transform ends, and
-  // not when one product's output is another's operand (the last pass of the
-  // one may run before the other's has read it).
-  bool late = tk == AOA_NTT && !(fuse & (kFuseKeyProduct | kFuseCombine));
+  // formed up front.  Not with the fused transform ends, and not when one
+  // product's output is another's operand (the last pass of the one may run
+  // before the other's has read it).
+  bool late = !(fuse & (kFuseKeyProduct | kFuseCombine));
   for (int x = 0; x < n && late; x++)
     for (int z = 0; z < n; z++) late = late && (x == z || (out[x] != a[z] && out[x] != b[z]));
   // small rings: five launches, the transforms as whole-limb clusters with the
@@ -318,10 +318,11 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
     }
     return;
   }
-  if (tk == AOA_DGT) {
+  if (late) {
+    if (tk == AOA_DGT) gi_tensor_d2_op(E, ptr, half, D2, n, m, st);
+    else tensor_d2_op(E, ptr, half, D2, n, m, st);
+  } else if (tk == AOA_DGT) {
     gi_tensor_batch_op(E, ptr, half, D, n, m, st);
-  } else if (late) {
-    tensor_d2_op(E, ptr, half, D2, n, m, st);
   } else {
     tensor_batch_op(E, ptr, half, D, n, m, st);
   }
@@ -337,7 +338,8 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
   modup(E, T, half, UB, (long)kl * N, n, level, st);
   if (tk == AOA_DGT) {
     xform(E, tk, UB, n, k, kl, kl, true, st);
-    gi_keyswitch_mul_batch_op(E, D2, half, UB, (long)kl * N, evk->d, KS, ks, n, m, st);
+    if (late) gi_keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, evk->d, KS + (long)m * N, ks, n, 0, st);
+    else gi_keyswitch_mul_batch_op(E, D2, half, UB, (long)kl * N, evk->d, KS, ks, n, m, st);
   } else if (fuse & kFuseKeyProduct) {
     NttIo io;                                  // special-limb transform with the key products fused
     io.epi.mode = kEpiKeyProduct;
@@ -356,15 +358,17 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
   xform(E, tk, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
   if (late) {
     if (do_rescale) {
-      hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
-      ntt_batch(E, U, 2 * n, level, 1, 1, false, st);
+      if (tk == AOA_DGT) gi_hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
+      else hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
+      xform(E, tk, U, 2 * n, level, 1, 1, false, st);
       rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st);
     } else {
       moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
     }
     const int nl = do_rescale ? level : m;
-    ntt_batch(E, Y, 2 * n, 0, nl, k, true, st);
-    hmult_finish_op(E, ptr, half, D2, evk->d, Y, outp, n, nl, do_rescale ? level : 0, st);
+    xform(E, tk, Y, 2 * n, 0, nl, k, true, st);
+    if (tk == AOA_DGT) gi_hmult_finish_op(E, ptr, half, D2, evk->d, Y, outp, n, nl, do_rescale ? level : 0, st);
+    else hmult_finish_op(E, ptr, half, D2, evk->d, Y, outp, n, nl, do_rescale ? level : 0, st);
   } else if (do_rescale) {
     ks_combine(E, U, N, D + (long)level * N, half, KS + (long)level * N, ks, nullptr, 0, 1, 2 * n, 0, st, level);
     xform(E, tk, U, 2 * n, level, 1, 1, false, st);

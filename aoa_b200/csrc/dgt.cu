@@ -214,17 +214,33 @@ __global__ void gi_keyswitch_mul(const uint64_t* xq, const uint64_t* xb, const u
   gi_keyswitch_at(xq, xb, key, key_half, k0, k1, nq, K, H, pc, n, blockIdx.y);
 }
 
-// the key products of op z = blockIdx.z: x at xq + z xq_stride (Q limbs) and
-// xb + z xb_stride (B limbs), k0 at k + z k_stride, k1 at k + (n + z) k_stride
+// the key products of ops z = blockIdx.z, blockIdx.z + gridDim.z, ...: x at xq +
+// z xq_stride (Q limbs) and xb + z xb_stride (B limbs), k0 at k + z k_stride, k1
+// at k + (nops + z) k_stride; a thread's key words are read once for its ops
 __global__ void gi_keyswitch_mul_batch(const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
                                        const uint64_t* key, long key_half, uint64_t* k, long k_stride, int nops,
                                        int nq, int K, int H, const PrimeConst* __restrict__ pc) {
   pdl_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
-  const int z = blockIdx.z;
-  gi_keyswitch_at(xq + z * xq_stride, xb + z * xb_stride, key, key_half, k + z * k_stride, k + (nops + z) * k_stride,
-                  nq, K, H, pc, n, blockIdx.y);
+  const int l = blockIdx.y, prime = l < nq ? l : K + (l - nq);
+  const long N = 2L * H;
+  const PrimeConst P = pc[prime];
+  const uint64_t* x = (l < nq ? xq + (long)l * N : xb + (long)(l - nq) * N) + n;
+  const long xs = l < nq ? xq_stride : xb_stride;
+  const uint64_t *pb = key + (long)prime * N + n, *pa = pb + key_half;
+  const uint64_t br = pb[0], bi = pb[H], ar = pa[0], ai = pa[H];
+  uint64_t* o = k + (long)l * N + n;
+  for (int z = blockIdx.z; z < nops; z += gridDim.z) {
+    const uint64_t xr = x[z * xs], xi = x[z * xs + H];
+    uint64_t r, i;
+    gi_mul_dev(xr, xi, br, bi, r, i, P);
+    o[z * k_stride] = r;
+    o[z * k_stride + H] = i;
+    gi_mul_dev(xr, xi, ar, ai, r, i, P);
+    o[(nops + z) * k_stride] = r;
+    o[(nops + z) * k_stride + H] = i;
+  }
 }
 
 // Reference GaussianInteger layout <-> planar GI limbs.
@@ -396,7 +412,8 @@ void gi_keyswitch_mul_batch_op(const Engine& E, const uint64_t* xq, long xq_stri
                                long xb_stride, const uint64_t* key, uint64_t* k, long k_stride, int n, int nq,
                                cudaStream_t st) {
   const dim3 g = gi_grid(E, nq + E.kl);
-  launch_pdl(gi_keyswitch_mul_batch, dim3(g.x, g.y, n), 256, 0, st, xq, xq_stride, xb, xb_stride, key,
+  const long want = (8L * E.num_sms + (long)g.x * g.y - 1) / ((long)g.x * g.y);   // about eight blocks per SM
+  launch_pdl(gi_keyswitch_mul_batch, dim3(g.x, g.y, (unsigned)std::max(1L, std::min((long)n, want))), 256, 0, st, xq, xq_stride, xb, xb_stride, key,
                                                               (long)(E.k + E.kl) * E.N, k, k_stride, n, nq, E.k,
                                                               (int)(E.N / 2), E.d_pc);
   AOA_CHECK_LAUNCH();

@@ -140,6 +140,107 @@ __global__ void __launch_bounds__(kThreads) galois_finish(const uint64_t* R, lon
   }
 }
 
+// ---- Gaussian integers (DGT contexts) ----------------------------------------------
+// A limb's planes re | im of H = N/2 words; one thread holds one Gaussian
+// integer.  A complex product sum takes one reduction per component for up to
+// four word products (4 q^2 in one Barrett step's range, as above).
+struct Gi {
+  uint64_t r, i;
+};
+__device__ __forceinline__ Gi gi_ld(const uint64_t* p, int H) { return Gi{p[0], p[H]}; }
+
+__device__ __forceinline__ Gi gi_mulmod(Gi a, Gi b, const PrimeConst& P) {
+  const uint64_t q = P.q;
+  const uint64_t s1 = mul_mod(a.r, b.r, P), s2 = mul_mod(a.i, b.i, P);
+  const uint64_t s3 = mul_mod(add_mod(a.r, a.i, q), add_mod(b.r, b.i, q), P);
+  return Gi{sub_mod(s1, s2, q), sub_mod(s3, add_mod(s1, s2, q), q)};
+}
+
+// a b + c d mod q
+__device__ __forceinline__ Gi gi_sum2(Gi a, Gi b, Gi c, Gi d, bool fit, const PrimeConst& P) {
+  const uint64_t q = P.q;
+  if (!fit) {
+    const Gi x = gi_mulmod(a, b, P), y = gi_mulmod(c, d, P);
+    return Gi{add_mod(x.r, y.r, q), add_mod(x.i, y.i, q)};
+  }
+  Gi s;
+  uint64_t lo = a.r * b.r, hi = __umul64hi(a.r, b.r);
+  mac_wide(lo, hi, q - a.i, b.i);
+  mac_wide(lo, hi, c.r, d.r);
+  mac_wide(lo, hi, q - c.i, d.i);
+  s.r = barrett_wide(lo, hi, q, P.bar_mu, (uint32_t)P.bar_sh);
+  lo = a.r * b.i;
+  hi = __umul64hi(a.r, b.i);
+  mac_wide(lo, hi, a.i, b.r);
+  mac_wide(lo, hi, c.r, d.i);
+  mac_wide(lo, hi, c.i, d.r);
+  s.i = barrett_wide(lo, hi, q, P.bar_mu, (uint32_t)P.bar_sh);
+  return s;
+}
+
+__device__ __forceinline__ Gi gi_add(Gi a, Gi b, uint64_t q) { return Gi{add_mod(a.r, b.r, q), add_mod(a.i, b.i, q)}; }
+__device__ __forceinline__ Gi gi_scale(Gi a, ShoupW w, uint64_t q) { return Gi{shoup(a.r, w, q), shoup(a.i, w, q)}; }
+
+__global__ void __launch_bounds__(kThreads) gi_tensor_d2(const __grid_constant__ CtPtrs ptr, long half, uint64_t* D2,
+                                                         const PrimeConst* pc, int log_n) {
+  pdl_begin();
+  const int H = 1 << (log_n - 1), z = blockIdx.z;
+  const PrimeConst P = pc[blockIdx.y];
+  const long off = ((long)blockIdx.y << log_n) + (long)blockIdx.x * kThreads + threadIdx.x;
+  const Gi a = gi_ld(ptr.a[z] + half + off, H), b = gi_ld(ptr.b[z] + half + off, H);
+  const Gi d = gi_mulmod(a, b, P);
+  D2[(long)z * half + off] = d.r;
+  D2[(long)z * half + off + H] = d.i;
+}
+
+// hmult_top and hmult_finish for Gaussian integers; MODE 0: the top limb (no
+// correction, out = U of stride N), 1: rescale, 2: without rescale
+template <int MODE>
+__global__ void __launch_bounds__(kThreads) gi_finish(const __grid_constant__ CtPtrs ptr, long half,
+                                                      const uint64_t* D2, const uint64_t* key, long key_half,
+                                                      const uint64_t* Y, const __grid_constant__ OutPtrs outp,
+                                                      uint64_t* U, int n, int limb0, const ShoupW* binv,
+                                                      const ShoupW* resc, const PrimeConst* pc, int log_n) {
+  pdl_begin();
+  const int H = 1 << (log_n - 1), i = limb0 + blockIdx.y;
+  const PrimeConst P = pc[i];
+  const uint64_t q = P.q;
+  const bool fit = sums_fit(P);
+  const ShoupW bi = binv[i], rs = MODE == 1 ? resc[i] : bi;
+  const long c = (long)blockIdx.x * kThreads + threadIdx.x, off = ((long)i << log_n) + c;
+  const Gi kb = gi_scale(gi_ld(key + off, H), bi, q), ka = gi_scale(gi_ld(key + key_half + off, H), bi, q);
+  for (int z = blockIdx.z; z < n; z += gridDim.z) {
+    const Gi a0 = gi_ld(ptr.a[z] + off, H), a1 = gi_ld(ptr.a[z] + half + off, H);
+    const Gi b0 = gi_ld(ptr.b[z] + off, H), b1 = gi_ld(ptr.b[z] + half + off, H);
+    const Gi d = gi_ld(D2 + (long)z * half + off, H);
+    Gi y0{0, 0}, y1{0, 0};
+    if (MODE) {
+      y0 = gi_ld(Y + (long)z * half + off, H);
+      y1 = gi_ld(Y + (long)(n + z) * half + off, H);
+    }
+    Gi c0 = gi_sum2(a0, b0, d, kb, fit, P);
+    Gi c1 = gi_add(gi_sum2(a0, b1, a1, b0, fit, P), gi_mulmod(d, ka, P), q);
+    uint64_t *o0 = MODE ? outp.p[z] + off : U + ((long)z << log_n) + c;
+    uint64_t *o1 = MODE ? outp.p[n + z] + off : U + ((long)(n + z) << log_n) + c;
+    if (MODE == 2) {
+      y0 = gi_scale(y0, bi, q);
+      y1 = gi_scale(y1, bi, q);
+    }
+    if (MODE) {
+      c0 = Gi{sub_mod(c0.r, y0.r, q), sub_mod(c0.i, y0.i, q)};
+      c1 = Gi{sub_mod(c1.r, y1.r, q), sub_mod(c1.i, y1.i, q)};
+    }
+    if (MODE == 1) {
+      c0 = gi_scale(c0, rs, q);
+      c1 = gi_scale(c1, rs, q);
+    }
+    o0[0] = c0.r;
+    o0[H] = c0.i;
+    o1[0] = c1.r;
+    o1[H] = c1.i;
+  }
+}
+
 // blocks over ops: one thread serves every op of the launch when the limbs
 // alone fill the chip, else the ops are spread so that about eight blocks per
 // SM are in flight
@@ -167,6 +268,26 @@ void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64
   const dim3 grid(E.N / (2 * kThreads), nlimbs, op_blocks(E, blocks, n));
   launch_pdl(resc ? hmult_finish<true> : hmult_finish<false>, grid, kThreads, 0, st, ptr, half, D2, key,
              (long)E.nprimes * E.N, Y, outp, n, E.rns.moddown_binv, resc, E.d_pc, E.log_n);
+}
+
+void gi_tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, int n, int nlimbs, cudaStream_t st) {
+  launch_pdl(gi_tensor_d2, dim3(E.N / (2 * kThreads), nlimbs, n), kThreads, 0, st, ptr, half, D2, E.d_pc, E.log_n);
+}
+
+void gi_hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+                     uint64_t* U, int n, int level, cudaStream_t st) {
+  launch_pdl(gi_finish<0>, dim3(E.N / (2 * kThreads), 1, n), kThreads, 0, st, ptr, half, D2, key,
+             (long)E.nprimes * E.N, nullptr, OutPtrs{}, U, n, level, E.rns.moddown_binv, nullptr, E.d_pc, E.log_n);
+}
+
+void gi_hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+                        const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level,
+                        cudaStream_t st) {
+  const ShoupW* resc = rescale_level > 0 ? E.rns.resc_inv + (long)rescale_level * E.k : nullptr;
+  const long blocks = E.N / (2 * kThreads) * nlimbs;
+  launch_pdl(resc ? gi_finish<1> : gi_finish<2>, dim3(E.N / (2 * kThreads), nlimbs, op_blocks(E, blocks, n)), kThreads,
+             0, st, ptr, half, D2, key, (long)E.nprimes * E.N, Y, outp, nullptr, n, 0, E.rns.moddown_binv, resc, E.d_pc,
+             E.log_n);
 }
 
 void galois_finish_op(const Engine& E, const uint64_t* R, long half, const KeyPtrs& keys, bool one_key,
