@@ -17,10 +17,16 @@
 //             (draw word 0, then the index: no ties), sign from draw bit
 //             32; the rest 0 (sample_hw: hw = 64; sample_Z0: hw = N/2)
 #include "aoa_internal.h"
+#include "async.cuh"
 
 using namespace aoa;
 
 namespace {
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 constexpr uint32_t kPhiloxM0 = 0xD2511F53u, kPhiloxM1 = 0xCD9E8D57u;
 constexpr uint32_t kPhiloxW0 = 0x9E3779B9u, kPhiloxW1 = 0xBB67AE85u;
@@ -51,6 +57,7 @@ __global__ void sample_uniform_kernel(uint64_t* out, long N, int nlimbs, int fir
 }
 
 __global__ void sample_gaussian_kernel(int64_t* out, long n, double sigma, uint64_t seed, uint64_t stream) {
+  pdl_begin();
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
     const uint4 r = philox((uint64_t)t, stream, seed);
     const uint64_t a = ((uint64_t)r.y << 32) | r.x, b = ((uint64_t)r.w << 32) | r.z;
@@ -61,47 +68,85 @@ __global__ void sample_gaussian_kernel(int64_t* out, long n, double sigma, uint6
   }
 }
 
-// One CTA: radix select of the hw smallest 64-bit keys (random word 0 in the
-// high 32 bits, the index in the low bits, so all keys differ), 8 bits per pass.
-constexpr int kSelThreads = 1024;
+// Radix select of the hw smallest 64-bit keys (random word 0 in the high 32
+// bits, the index in the low bits, so all keys differ) by one cluster of eight
+// CTAs, 11 bits a pass: every CTA counts its share of the keys, and after a
+// cluster barrier each sums the eight histograms through distributed shared
+// memory and finds the same digit.  The passes end when every key under the
+// prefix is taken, as a rule after the random word's three.  The keys are drawn
+// once (up to kSelCache per CTA) while the stream's previous kernel ends.  One
+// CTA drawing every key again in each of eight 8-bit passes took 76 us for
+// 2^14 keys.
+constexpr int kSelThreads = 1024, kSelCtas = 8, kSelBins = 2048;
+constexpr long kSelCache = 16384;
 
-__global__ void __launch_bounds__(kSelThreads) sample_ternary_kernel(int64_t* out, long n, long hw, uint64_t seed,
-                                                                      uint64_t stream) {
-  __shared__ unsigned hist[256];
-  __shared__ uint64_t prefix_s, mask_s;
-  __shared__ long need_s;
-  auto key_of = [&](long i) { return ((uint64_t)philox((uint64_t)i, stream, seed).x << 32) | (uint64_t)i; };
-  if (threadIdx.x == 0) {
-    prefix_s = 0;
-    mask_s = 0;
-    need_s = hw;                       // keys still to take below the current prefix
-  }
-  __syncthreads();
-  for (int shift = 56; shift >= 0; shift -= 8) {
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
+__global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
+sample_ternary_kernel(int64_t* out, long n, long hw, uint64_t seed, uint64_t stream) {
+  extern __shared__ uint64_t words[];        // random word 0, sign in bit 32
+  __shared__ __align__(8) unsigned hist[kSelBins];
+  __shared__ unsigned warp_sum[32];
+  __shared__ unsigned found_bin, found_need, found_count;
+  const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+  const long chunk = (n + kSelCtas - 1) / kSelCtas;
+  const long i0 = blockIdx.x * chunk, cnt = max(0L, min(chunk, n - i0));
+  const bool cached = chunk <= kSelCache;
+  auto draw = [&](long t) {
+    const uint4 r = philox((uint64_t)(i0 + t), stream, seed);
+    return (uint64_t)r.x | ((uint64_t)(r.y & 1) << 32);
+  };
+  auto word = [&](long t) { return cached ? words[t] : draw(t); };
+  if (cached)
+    for (long t = tid; t < cnt; t += kSelThreads) words[t] = draw(t);   // read by the same thread only
+  uint64_t prefix = 0, mask = 0, kth = 0;
+  unsigned need = (unsigned)hw;              // keys still to take under the current prefix
+  const uint32_t h_addr = smem_u32(hist);
+  constexpr int kShift[6] = {53, 42, 32, 21, 10, 0};
+  for (int d = 0; d < 6 && need > 0; d++) {
+    const int shift = kShift[d], width = d % 3 == 2 ? 10 : 11;
+    for (int i = tid; i < kSelBins; i += kSelThreads) hist[i] = 0;
     __syncthreads();
-    const uint64_t prefix = prefix_s, mask = mask_s;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) {
-      const uint64_t k = key_of(i);
-      if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & 255], 1u);
+    for (long t = tid; t < cnt; t += kSelThreads) {
+      const uint64_t k = (word(t) << 32) | (uint64_t)(i0 + t);
+      if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & ((1u << width) - 1)], 1u);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      long need = need_s;
-      int b = 0;
-      for (; b < 255 && (long)hist[b] < need; b++) need -= hist[b];
-      prefix_s = prefix | ((uint64_t)b << shift);
-      mask_s = mask | ((uint64_t)255 << shift);
-      need_s = need;
+    cluster_barrier();
+    unsigned c0 = 0, c1 = 0;                 // bins 2 tid, 2 tid + 1 of the whole cluster
+    for (int r = 0; r < kSelCtas; r++) {
+      uint32_t a, x, y;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(h_addr + tid * 8), "r"(r));
+      asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(a));
+      c0 += x;
+      c1 += y;
     }
+    unsigned incl = c0 + c1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned v = __shfl_up_sync(~0u, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
     __syncthreads();
+    unsigned before = incl - c0 - c1;        // keys in lower bins
+    for (int w = 0; w < warp; w++) before += warp_sum[w];
+    if (before < need && need <= before + c0) {
+      found_bin = 2 * tid;
+      found_need = need - before;
+      found_count = c0;
+    } else if (before + c0 < need && need <= before + c0 + c1) {
+      found_bin = 2 * tid + 1;
+      found_need = need - before - c0;
+      found_count = c1;
+    }
+    cluster_barrier();                       // every histogram is read; the digit is visible
+    prefix |= (uint64_t)found_bin << shift;
+    mask |= (uint64_t)((1u << width) - 1) << shift;
+    kth = prefix | ((1ull << shift) - 1);
+    need = found_need;
+    if (found_count == need) break;          // every key under the prefix is taken
   }
-  // prefix_s is now the hw-th smallest key (keys are distinct)
-  const uint64_t kth = prefix_s;
-  for (long i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint4 r = philox((uint64_t)i, stream, seed);
-    const uint64_t k = ((uint64_t)r.x << 32) | (uint64_t)i;
-    out[i] = (hw > 0 && k <= kth) ? ((r.y & 1) ? -1 : 1) : 0;
+  pdl_begin();
+  for (long t = tid; t < cnt; t += kSelThreads) {
+    const uint64_t w = word(t), k = (w << 32) | (uint64_t)(i0 + t);
+    out[i0 + t] = hw > 0 && k <= kth ? ((w >> 32) ? -1 : 1) : 0;
   }
 }
 
@@ -151,8 +196,7 @@ int aoa_sample_gaussian(aoa_ctx* c, int64_t* d_out, long n, double sigma, uint64
   if (!c || !d_out || n < 0 || !(sigma >= 0)) return fail(AOA_ERR_BAD_PARAM, "bad argument");
   return guarded([&] {
     if (n == 0) return;
-    sample_gaussian_kernel<<<2 * c->c.E->num_sms, 256, 0, c->c.stream>>>(d_out, n, sigma, seed, stream);
-    note_launch();
+    launch_pdl(sample_gaussian_kernel, 2 * c->c.E->num_sms, 256, 0, c->c.stream, d_out, n, sigma, seed, stream);
     AOA_CHECK_LAUNCH();
   });
 }
@@ -161,8 +205,11 @@ int aoa_sample_ternary(aoa_ctx* c, int64_t* d_out, long n, long hw, uint64_t see
   if (!c || !d_out || n < 0 || hw < 0 || hw > n || n > (1L << 31)) return fail(AOA_ERR_BAD_PARAM, "bad argument");
   return guarded([&] {
     if (n == 0) return;
-    sample_ternary_kernel<<<1, kSelThreads, 0, c->c.stream>>>(d_out, n, hw, seed, stream);
-    note_launch();
+    const long chunk = (n + kSelCtas - 1) / kSelCtas;
+    const size_t smem = chunk <= kSelCache ? (size_t)chunk * 8 : 0;
+    AOA_CUDA(cudaFuncSetAttribute(sample_ternary_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kSelCache * 8)));
+    launch_pdl(sample_ternary_kernel, kSelCtas, kSelThreads, smem, c->c.stream, d_out, n, hw, seed, stream);
     AOA_CHECK_LAUNCH();
   });
 }
