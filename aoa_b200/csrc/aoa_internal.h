@@ -131,10 +131,9 @@ struct Engine {
   // Device error word: kernels OR in kErr* bits instead of trapping (a bounded
   // wait that expired, ...); aoa_ctx_sync reads and clears it.
   unsigned* d_err = nullptr;
-  // Encoder tables: ksi[j] = exp(2 pi i j / M) for j <= M = 2N, as FP64 pairs
-  // computed on the host; rot[j] = 5^j mod M for j < N/2.
-  double2* d_ksi = nullptr;
-  uint32_t* d_rot = nullptr;
+  // Encoder tables: the roots of each FFT stage in order (build_encoder_tables)
+  double2* d_roots = nullptr;
+  double2* d_roots_inv = nullptr;
   // DGT (folded Gaussian-integer transform of length N/2): cyclic merged
   // tables per prime, constants with N/2 inverses, and the twist by the
   // powers of a root r of i (r^(N/2) = i).  The twist tables hold r^n = c + di
@@ -376,6 +375,7 @@ void tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, i
 void hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key, uint64_t* U,
                   int n, int level, cudaStream_t st);
 void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
+                     const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
 // the same with Gaussian-integer products (DGT domain, planar limbs)
 void gi_tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, int n, int nlimbs, cudaStream_t st);
 void gi_hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
@@ -383,7 +383,6 @@ void gi_hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64
 void gi_hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
                         const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level,
                         cudaStream_t st);
-                     const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
 void galois_finish_op(const Engine& E, const uint64_t* R, long half, const KeyPtrs& keys, bool one_key,
                       const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, bool add, cudaStream_t st);
 void automorph_ntt_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* out, int n,

@@ -51,25 +51,21 @@ __device__ __forceinline__ unsigned bitrev_bits(unsigned x, int bits) {
   return bits ? __brev(x) >> (32 - bits) : 0u;
 }
 
-// Inverse-FFT butterfly at (a, b = a + lenh) with in-group index j
-// (fftSpecialInv: u = x + y, v = (x - y) * ksi[(lenq - rot[j] % lenq) * M / lenq]).
-__device__ __forceinline__ void inv_bf(double2& x, double2& y, unsigned j, unsigned len, const double2* ksi,
-                                       const uint32_t* rot, unsigned M) {
-  const unsigned lenq = len << 2;
-  const unsigned idx = (lenq - (rot[j] & (lenq - 1))) * (M / lenq);
+// Butterflies of span len at in-group index j; the roots of a stage sit in order
+// at w[len / 2 + j] (build_encoder_tables), so that neighbouring threads read
+// neighbouring roots: through the rotation group a root took two dependent
+// gathers, most of a stage's time.
+// Inverse (fftSpecialInv): u = x + y, v = (x - y) * root.
+__device__ __forceinline__ void inv_bf(double2& x, double2& y, double2 w) {
   const double2 u = c_add(x, y);
-  const double2 v = c_mul(c_sub(x, y), ksi[idx]);
+  const double2 v = c_mul(c_sub(x, y), w);
   x = u;
   y = v;
 }
 
-// Forward-FFT butterfly (fftSpecial: v = y * ksi[(rot[j] % lenq) * M / lenq];
-// x, y = x + v, x - v).
-__device__ __forceinline__ void fwd_bf(double2& x, double2& y, unsigned j, unsigned len, const double2* ksi,
-                                       const uint32_t* rot, unsigned M) {
-  const unsigned lenq = len << 2;
-  const unsigned idx = (rot[j] & (lenq - 1)) * (M / lenq);
-  const double2 v = c_mul(y, ksi[idx]);
+// Forward (fftSpecial): v = y * root; x, y = x + v, x - v.
+__device__ __forceinline__ void fwd_bf(double2& x, double2& y, double2 w) {
+  const double2 v = c_mul(y, w);
   const double2 u = x;
   x = c_add(u, v);
   y = c_sub(u, v);
@@ -77,8 +73,7 @@ __device__ __forceinline__ void fwd_bf(double2& x, double2& y, unsigned j, unsig
 
 // One stage of span `len` over the whole vector: thread t handles butterfly t.
 template <bool INV>
-__global__ void fft_stage(double2* v, unsigned size, unsigned len, const double2* __restrict__ ksi,
-                          const uint32_t* __restrict__ rot, unsigned M) {
+__global__ void fft_stage(double2* v, unsigned size, unsigned len, const double2* __restrict__ roots) {
   pdl_begin();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= size / 2) return;
@@ -86,15 +81,14 @@ __global__ void fft_stage(double2* v, unsigned size, unsigned len, const double2
   const unsigned j = t % lenh;
   const unsigned a = (t / lenh) * len + j;
   double2 x = v[a], y = v[a + lenh];
-  if (INV) inv_bf(x, y, j, len, ksi, rot, M);
-  else fwd_bf(x, y, j, len, ksi, rot, M);
+  if (INV) inv_bf(x, y, roots[lenh + j]);
+  else fwd_bf(x, y, roots[lenh + j]);
   v[a] = x;
   v[a + lenh] = y;
 }
 
 // Inverse stages len = tile .. 2 on one tile of `tile` consecutive entries.
-__global__ void fft_inv_tile(double2* v, unsigned tile, const double2* __restrict__ ksi,
-                             const uint32_t* __restrict__ rot, unsigned M) {
+__global__ void fft_inv_tile(double2* v, unsigned tile, const double2* __restrict__ roots) {
   pdl_begin();
   extern __shared__ double2 sv[];
   double2* g = v + (size_t)blockIdx.x * tile;
@@ -105,7 +99,7 @@ __global__ void fft_inv_tile(double2* v, unsigned tile, const double2* __restric
     for (unsigned t = threadIdx.x; t < tile / 2; t += blockDim.x) {
       const unsigned j = t % lenh;
       const unsigned a = (t / lenh) * len + j;
-      inv_bf(sv[a], sv[a + lenh], j, len, ksi, rot, M);
+      inv_bf(sv[a], sv[a + lenh], roots[lenh + j]);
     }
     __syncthreads();
   }
@@ -121,8 +115,7 @@ __device__ __forceinline__ double adjust_scale(uint64_t x, uint64_t p, double fa
 // tile, then forward stages len = 2 .. tile in shared memory.
 __global__ void fft_fwd_tile_from_message(double2* v, const uint64_t* __restrict__ m0, uint64_t p, double factor,
                                           int log_size, unsigned tile, unsigned gap, unsigned half_n,
-                                          const double2* __restrict__ ksi, const uint32_t* __restrict__ rot,
-                                          unsigned M) {
+                                          const double2* __restrict__ roots) {
   pdl_begin();
   extern __shared__ double2 sv[];
   const unsigned base = blockIdx.x * tile;
@@ -137,7 +130,7 @@ __global__ void fft_fwd_tile_from_message(double2* v, const uint64_t* __restrict
     for (unsigned t = threadIdx.x; t < tile / 2; t += blockDim.x) {
       const unsigned j = t % lenh;
       const unsigned a = (t / lenh) * len + j;
-      fwd_bf(sv[a], sv[a + lenh], j, len, ksi, rot, M);
+      fwd_bf(sv[a], sv[a + lenh], roots[lenh + j]);
     }
     __syncthreads();
   }
@@ -233,16 +226,14 @@ int aoa_encode(aoa_ctx* c, const double* host_vals, int filled, int empty, uint6
     if (filled)
       AOA_CUDA(cudaMemcpyAsync(v, host_vals, (size_t)filled * 16, cudaMemcpyHostToDevice, C.stream));
     if (empty) AOA_CUDA(cudaMemsetAsync(v + filled, 0, (size_t)empty * 16, C.stream));
-    const unsigned M = (unsigned)(2 * E.N);
     const unsigned tile = (unsigned)std::min<long>(slots, kFftTile);
     for (long len = slots; len > (long)tile; len >>= 1) {
-      launch_pdl(fft_stage<true>, (unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream, v, (unsigned)slots, (unsigned)len,
-                                                                                  E.d_ksi, E.d_rot, M);
+      launch_pdl(fft_stage<true>, (unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream, v, (unsigned)slots, (unsigned)len, E.d_roots_inv);
       AOA_CHECK_LAUNCH();
     }
     if (tile >= 2) {
       launch_pdl(fft_inv_tile, (unsigned)(slots / tile), std::min(tile / 2, 1024u), tile * sizeof(double2), C.stream, 
-          v, tile, E.d_ksi, E.d_rot, M);
+          v, tile, E.d_roots_inv);
       AOA_CHECK_LAUNCH();
     }
     dim3 grid((unsigned)((E.N + 255) / 256), (unsigned)nlimbs);
@@ -274,15 +265,12 @@ int aoa_decode(aoa_ctx* c, const uint64_t* d_m, int domain, int slots, uint64_t 
       xform(E, domain, limb, 1, 0, 1, 1, false, C.stream);
       m0 = limb;
     }
-    const unsigned M = (unsigned)(2 * E.N);
     const unsigned tile = (unsigned)std::min<int>(slots, kFftTile);
     launch_pdl(fft_fwd_tile_from_message, (unsigned)(slots / tile), std::max(1u, std::min(tile / 2, 1024u)), tile * sizeof(double2), C.stream, 
-        v, m0, E.primes[0], (double)scale, log_size, tile, (unsigned)(E.N / 2 / slots), (unsigned)(E.N / 2), E.d_ksi,
-        E.d_rot, M);
+        v, m0, E.primes[0], (double)scale, log_size, tile, (unsigned)(E.N / 2 / slots), (unsigned)(E.N / 2), E.d_roots);
     AOA_CHECK_LAUNCH();
     for (long len = 2L * tile; len <= slots; len <<= 1) {
-      launch_pdl(fft_stage<false>, (unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream, v, (unsigned)slots, (unsigned)len,
-                                                                                   E.d_ksi, E.d_rot, M);
+      launch_pdl(fft_stage<false>, (unsigned)((slots / 2 + 255) / 256), 256, 0, C.stream, v, (unsigned)slots, (unsigned)len, E.d_roots);
       AOA_CHECK_LAUNCH();
     }
     AOA_CUDA(cudaMemcpyAsync(host_vals, v, (size_t)slots * 16, cudaMemcpyDeviceToHost, C.stream));

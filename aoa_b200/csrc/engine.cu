@@ -108,24 +108,30 @@ static void build_prime_tables(Engine& E) {
 
 // Encoder tables (the reference computes them on the host per call,
 // aoa-ntt src/ckks/encoder.cu:33-124).  ksi[j] = (cos(2 pi j / M), sin(2 pi j / M))
-// with M = 2N, evaluated by the host libm exactly as written so that the
-// device FFT uses the same doubles; rot[j] = 5^j mod M.
+// with M = 2N, evaluated by the host libm exactly as written so that the device
+// FFT uses the same doubles; rot[j] = 5^j mod M.  The stage of span len multiplies
+// by ksi[(rot[j] mod 4 len) M / (4 len)] at in-group index j (fftSpecial), by the
+// conjugate index in the inverse: kept in that order at roots[len / 2 + j].
 static void build_encoder_tables(Engine& E) {
   const long M = 2 * E.N;
-  std::vector<double2> ksi(M + 1);
+  std::vector<double2> ksi(M + 1), fwd(std::max<long>(1, E.N / 2)), inv(fwd.size());
   for (long j = 0; j < M; ++j) {
     const double angle = 2.0 * M_PI * j / M;
     ksi[j] = make_double2(cos(angle), sin(angle));
   }
   ksi[M] = ksi[0];
-  std::vector<uint32_t> rot(std::max<long>(1, E.N / 2));
-  uint64_t v = 1;
-  for (long j = 0; j < E.N / 2; ++j) {
-    rot[j] = (uint32_t)v;
-    v = (v * 5) % (uint64_t)M;
+  for (long len = 2; len <= E.N / 2; len <<= 1) {
+    const long lenh = len >> 1, lenq = len << 2;
+    uint64_t v = 1;
+    for (long j = 0; j < lenh; ++j) {
+      const long r = (long)(v & (uint64_t)(lenq - 1));
+      fwd[lenh + j] = ksi[r * (M / lenq)];
+      inv[lenh + j] = ksi[(lenq - r) * (M / lenq)];
+      v = (v * 5) % (uint64_t)M;
+    }
   }
-  E.d_ksi = dev_upload(E, ksi);
-  E.d_rot = dev_upload(E, rot);
+  E.d_roots = dev_upload(E, fwd);
+  E.d_roots_inv = dev_upload(E, inv);
 }
 
 // Basis-conversion and rescale constants (manager.cu:566-759).
