@@ -9,11 +9,6 @@ AOA_NTT_KIND(extern, kButterflyCanonical)
 AOA_NTT_KIND(extern, kButterflyLazy)
 AOA_NTT_KIND(extern, kButterflyLazyQ1)
 
-// the inverse column pass keeps the general remainder on primes
-// q = 1 mod 2^32: with the short one it measured 3% slower (more carries on
-// the multiply pipe in its Gentleman-Sande butterflies)
-static constexpr int inverse_cols(int kind) { return kind == kButterflyLazyQ1 ? kButterflyLazy : kind; }
-
 void ntt_init(Engine& E) {
   allow_kind<kButterflyCanonical>();
   allow_kind<kButterflyLazy>();
@@ -186,7 +181,7 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
 #define AOA_KIND(K)                                                                   \
   case K:                                                                             \
     if (forward) { run_cols<K>(E, first, true, st); run_rows<K>(E, b, true, st, epi); }  \
-    else { run_rows<K>(E, first, false, st, no_epi); run_cols<inverse_cols(K)>(E, b, false, st); }     \
+    else { run_rows<K>(E, first, false, st, no_epi); run_cols<K>(E, b, false, st); }     \
     break;
       AOA_KIND(kButterflyCanonical) AOA_KIND(kButterflyLazy) AOA_KIND(kButterflyLazyQ1)
 #undef AOA_KIND

@@ -64,7 +64,7 @@ struct Bf<kButterflyCanonical> {
     x = add_mod(U, V, q);
     y = sub_mod(U, V, q);
   }
-  static __device__ __forceinline__ void gs(uint64_t& x, uint64_t& y, ShoupW w, uint64_t q) {
+  static __device__ __forceinline__ void gs(uint64_t& x, uint64_t& y, ShoupW w, uint64_t q, int) {
     uint64_t U = x, V = y;
     x = add_mod(U, V, q);
     y = shoup(sub_mod(U, V, q), w, q);
@@ -87,8 +87,12 @@ struct Bf<kButterflyCanonical> {
 // no faster than the compiler's lowering).  Forward values stay below 16q
 // (< 2^64): a reducing stage (even stage index within its pass) maps [0, 16q)
 // to [0, 12q) (U reduced by 8q), the stage after it maps [0, 12q) to
-// [0, 16q), up to the 2^32 that csub_hi may leave.  Inverse values stay in
-// [0, 4q), reduced at every stage.
+// [0, 16q), up to the 2^32 that csub_hi may leave.  Inverse values stay below
+// 8q: a sum is reduced by 8q only where its terms may have reached 8q, not
+// where the stage before wrote both of them as products (inv_bound): 64 x 30
+// limbs at 2^16, forward + inverse with copies, 3200 -> 3130 us, and with the
+// short remainder in the inverse column pass of primes q = 1 mod 2^32 as well
+// (whose carries had cost more than it saved there) 3102 us.
 template <int KIND>
 struct Bf {
   static __device__ __forceinline__ uint64_t mulw(uint64_t y, ShoupW w, uint64_t q) {   // [0, 4q)
@@ -136,18 +140,18 @@ struct Bf {
     x = U + V;                                  // [0, 12q) if red, else [0, 16q)
     y = U - V + q4;                             // likewise
   }
-  // inputs and outputs in [0, 4q)
-  static __device__ __forceinline__ void gs(uint64_t& x, uint64_t& y, ShoupW w, uint64_t q) {
-    const uint64_t q4 = q << 2;
+  // inputs in [0, bound q), bound 4 or 8 (a compile-time constant after
+  // unrolling): x in [0, 8q), y in [0, 4q)
+  static __device__ __forceinline__ void gs(uint64_t& x, uint64_t& y, ShoupW w, uint64_t q, int bound) {
     const uint64_t U = x, V = y;
-    x = csub(U + V, q4);
-    y = mulw(U - V + q4, w, q);
+    x = bound > 4 ? csub(U + V, q << 3) : U + V;
+    y = mulw(U - V + q * bound, w, q);
   }
-  // final inverse stage with N^-1 folded in: outputs in [0, q)
+  // final inverse stage with N^-1 folded in: inputs in [0, 8q), outputs in [0, q)
   static __device__ __forceinline__ void gs_last(uint64_t& x, uint64_t& y, ShoupW n0, ShoupW n1, uint64_t q) {
     const uint64_t U = x, V = y;
     const uint64_t a = mulw(U + V, n0, q);
-    const uint64_t b = mulw(U - V + (q << 2), n1, q);
+    const uint64_t b = mulw(U - V + (q << 3), n1, q);
     x = csub(csub(a, q << 1), q);
     y = csub(csub(b, q << 1), q);
   }
@@ -233,6 +237,12 @@ __device__ __forceinline__ void fwd_low_s(uint64_t (&u)[Sub<LOG_S>::L], uint32_t
 }
 
 // ---- inverse (Gentleman-Sande) -------------------------------------------
+// Bound (in q) of the pair at local index h before the i-th stage of a round
+// that starts below `entry` q: both were products (4) or both sums (8) in the
+// stage before, which paired indexes differing in bit i - 1.
+__device__ __forceinline__ constexpr int inv_bound(int i, int h, int entry) {
+  return i == 0 ? entry : (h >> (i - 1)) & 1 ? 4 : 8;
+}
 
 template <int LOG_S, int LAZY, bool PERM = false>
 __device__ __forceinline__ void inv_low_s(uint64_t (&u)[Sub<LOG_S>::L], uint32_t itw, uint32_t hi, uint64_t q) {
@@ -244,7 +254,7 @@ __device__ __forceinline__ void inv_low_s(uint64_t (&u)[Sub<LOG_S>::L], uint32_t
     for (int l = 0; l < D::L; l++) {
       if (l & span) continue;
       const ShoupW w = ldsw(itw + 16 * low_tw_index<LOG_S, PERM>(i, hi, l >> (i + 1)));
-      Bf<LAZY>::gs(u[l], u[l + span], w, q);
+      Bf<LAZY>::gs(u[l], u[l + span], w, q, inv_bound(i, l, 8));
     }
   }
 }
@@ -265,7 +275,7 @@ __device__ __forceinline__ void inv_high_s(uint64_t (&v)[Sub<LOG_S>::E], uint32_
         Bf<LAZY>::gs_last(v[h], v[h + span], ninv, ninv_w1, q);
       } else {
         const ShoupW w = ldsw(itw + 16 * ((1 << (D::HI - 1 - i)) + (h >> (i + 1))));
-        Bf<LAZY>::gs(v[h], v[h + span], w, q);
+        Bf<LAZY>::gs(v[h], v[h + span], w, q, inv_bound(i, h, 8));
       }
     }
   }
@@ -317,7 +327,8 @@ __device__ __forceinline__ void inv_low_r(uint64_t (&u)[Sub<LOG_S>::L], const Sh
 #pragma unroll
     for (int l = 0; l < D::L; l++) {
       if (l & span) continue;
-      Bf<LAZY>::gs(u[l], u[l + span], w[(1 << (D::LO - 1 - i)) - 1 + (l >> (i + 1))], q);
+      Bf<LAZY>::gs(u[l], u[l + span], w[(1 << (D::LO - 1 - i)) - 1 + (l >> (i + 1))], q,
+                   inv_bound(i, l, 4));   // the transform's first stages
     }
   }
 }
@@ -845,7 +856,7 @@ ntt_rows(NttBatch b, const __grid_constant__ NttEpi epi) {
         for (int h = 0; h < D::E; h++) {
           if (h & span) continue;
           const ShoupW wv = ldsw(st1 + 16 * ((1 << (D::HI - 1 - i)) - 1 + (h >> (i + 1))));
-          Bf<LAZY>::gs(v[h], v[h + span], wv, q);
+          Bf<LAZY>::gs(v[h], v[h + span], wv, q, inv_bound(i, h, 8));
         }
       }
 #pragma unroll

@@ -215,7 +215,7 @@ __device__ __forceinline__ void limb_fwd(const LimbSmem& s, uint32_t rank, uint6
   }
 }
 
-// The row tile (words below 4q on lazy primes) to the finished inverse limb at
+// The row tile (words below 8q on lazy primes) to the finished inverse limb at
 // x.  WAIT: the barrier that every CTA of the cluster arrives at when it starts
 // is still to be waited for (a forward transform has done so, and its own
 // barrier has every column tile read).
@@ -231,7 +231,7 @@ __device__ __forceinline__ void limb_inv(const LimbSmem& s, uint32_t rank, uint6
       const int hi = G % (L::C / 2), r = G / (L::C / 2);
       const uint32_t a = s.row + (r * L::C + row_word(2 * hi)) * 8, b = s.row + (r * L::C + row_word(2 * hi + 1)) * 8;
       uint64_t u = lds64(a), y = lds64(b);
-      Bf<KIND>::gs(u, y, ldsw(tr + (L::RW * ((1 << st) - 1) + (r << st) + hi) * 16), q);
+      Bf<KIND>::gs(u, y, ldsw(tr + (L::RW * ((1 << st) - 1) + (r << st) + hi) * 16), q, 8);
       sts64(a, u);
       sts64(b, y);
     }
@@ -250,10 +250,10 @@ __device__ __forceinline__ void limb_inv(const LimbSmem& s, uint32_t rank, uint6
       for (int j = 0; j < 4; j++) v[j] = lds64(a + row_word(i0 + j * d) * 8);
       const ShoupW w0 = ldsw(tr + (L::RW * ((1 << st) - 1) + (r << st) + hi) * 16);
       const uint32_t t1 = tr + (L::RW * ((2 << st) - 1) + (r << (st + 1)) + 2 * hi) * 16;
-      Bf<KIND>::gs(v[0], v[1], ldsw(t1), q);
-      Bf<KIND>::gs(v[2], v[3], ldsw(t1 + 16), q);
-      Bf<KIND>::gs(v[0], v[2], w0, q);
-      Bf<KIND>::gs(v[1], v[3], w0, q);
+      Bf<KIND>::gs(v[0], v[1], ldsw(t1), q, 8);
+      Bf<KIND>::gs(v[2], v[3], ldsw(t1 + 16), q, 8);
+      Bf<KIND>::gs(v[0], v[2], w0, q, 8);
+      Bf<KIND>::gs(v[1], v[3], w0, q, 8);
       if (st) {
 #pragma unroll
         for (int j = 0; j < 4; j++) sts64(a + row_word(i0 + j * d) * 8, v[j]);
@@ -280,12 +280,12 @@ __device__ __forceinline__ void limb_inv(const LimbSmem& s, uint32_t rank, uint6
 #pragma unroll
       for (int j = 0; j < 4; j++) v[j] = lds64(a + j * step);
       const uint32_t t = s.ti + (2 << st) * 16 + 2 * hi * 16;
-      Bf<KIND>::gs(v[0], v[1], ldsw(t), q);
-      Bf<KIND>::gs(v[2], v[3], ldsw(t + 16), q);
+      Bf<KIND>::gs(v[0], v[1], ldsw(t), q, 8);
+      Bf<KIND>::gs(v[2], v[3], ldsw(t + 16), q, 8);
       if (st) {
         const ShoupW w0 = ldsw(s.ti + ((1 << st) + hi) * 16);
-        Bf<KIND>::gs(v[0], v[2], w0, q);
-        Bf<KIND>::gs(v[1], v[3], w0, q);
+        Bf<KIND>::gs(v[0], v[2], w0, q, 8);
+        Bf<KIND>::gs(v[1], v[3], w0, q, 8);
 #pragma unroll
         for (int j = 0; j < 4; j++) sts64(a + j * step, v[j]);
       } else {                             // the last stage, with N^-1
