@@ -89,13 +89,16 @@ struct RnsTables {
   // ModUp at level l (fast_conv_Q_to_B, manager.cu:180-223):
   //   modup_inv[l*k + i]          = (Q_l/q_i)^-1 mod q_i        (Shoup form)
   //   modup_hat[(l*k + i)*kl + j] = (Q_l/q_i) mod b_j
+  //   modup_inv_n, moddown_inv_n: times N^-1, for unscaled inputs
   ShoupW* modup_inv = nullptr;
+  ShoupW* modup_inv_n = nullptr;
   uint64_t* modup_hat = nullptr;
   // ModDown (fast_conv_B_to_Q, manager.cu:312-341):
   //   moddown_inv[j]         = ((B/b_j) mod b_j)^-1            (Shoup form)
   //   moddown_hat[j*k + i]   = (B/b_j) mod q_i
   //   moddown_binv[i]        = (B mod q_i)^-1                 (Shoup form)
   ShoupW* moddown_inv = nullptr;
+  ShoupW* moddown_inv_n = nullptr;
   uint64_t* moddown_hat = nullptr;
   ShoupW* moddown_binv = nullptr;
   // Rescale (ckks_rescale, manager.cu:90-118): resc_inv[l*k + i] = q_l^-1 mod q_i
@@ -251,7 +254,10 @@ struct NttTables {
 };
 // Fused ends of a limb transform.  NttIo::src: the first pass reads item
 // (p, l) from src + p * src_poly_stride + l * N instead of the data (an
-// out-of-place transform; the data is written).  NttIo::epi: what the last
+// out-of-place transform; the data is written).  NttIo::unscaled: an inverse
+// without its factor N^-1 and last reduction (words below 16 q), for the basis
+// conversions, whose first product takes both up (`unscaled` there): one of 4.5
+// products per coefficient of the inverse column pass saved.  NttIo::epi: what the last
 // pass of a FORWARD transform does with the finished value v of coefficient c
 // of item (p, l) under prime pr (p counts from the first poly of the call):
 //   kEpiStore       data = v
@@ -284,6 +290,7 @@ struct NttEpi {
 struct NttIo {
   const uint64_t* src = nullptr;
   long src_poly_stride = 0;
+  bool unscaled = false;
   NttEpi epi;
 };
 void ntt_init(Engine& E);
@@ -300,14 +307,15 @@ void ntt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int
 void limb_init(const Engine& E);
 bool limb_serves(const Engine& E, int log_n, long items, bool fused);
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
-                    long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, cudaStream_t st);
-// D2 + z half = a1 b1 and T + z half = its inverse transform, op z
+                    long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, bool unscaled,
+                    cudaStream_t st);
+// D2 + z half = a1 b1 and T + z half = its unscaled inverse transform, op z
 void limb_tensor_inv(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, uint64_t* T, int n, int nlimbs,
                      cudaStream_t st);
-// R = permuted [c0 | c1] of every op, T = the inverse transform of the permuted c1
+// R = permuted [c0 | c1] of every op, T = the unscaled inverse of the permuted c1
 void limb_galois_inv(const Engine& E, const CtPtrs& ptr, const GaloisList& g, long half, uint64_t* R, uint64_t* T,
                      int n, int nlimbs, cudaStream_t st);
-// special limbs: KS + (part n + z) ks_stride = inverse(forward(UB of op z) key part); with ptr also
+// special limbs: KS + (part n + z) ks_stride = unscaled inverse(forward(UB of op z) key part); with ptr also
 // U + (part n + z) N = inverse of the top limb of d + d2 key B^-1
 void limb_key(const Engine& E, const uint64_t* UB, uint64_t* KS, long ks_stride, const KeyPtrs& keys, int n,
               const CtPtrs* ptr, long half, const uint64_t* D2, uint64_t* U, int level, cudaStream_t st);
@@ -319,16 +327,17 @@ void limb_galois_finish(const Engine& E, uint64_t* Y, const uint64_t* R, long ha
 
 // rns.cu
 void rns_init(Engine& E);
+// unscaled: the input limbs lack N^-1 and are any words congruent to them (NttIo::unscaled)
 void modup(const Engine& E, const uint64_t* in, long in_stride, uint64_t* out_b, long out_stride,
-           int npolys, int level, cudaStream_t st);
+           int npolys, int level, cudaStream_t st, bool unscaled = false);
 void moddown(const Engine& E, const uint64_t* in_q, const uint64_t* in_b, long in_stride, uint64_t* out,
              long out_stride, int npolys, int level, cudaStream_t st);
 void rescale(const Engine& E, uint64_t* d, long poly_stride, int npolys, int level, cudaStream_t st);
 void moddown_conv(const Engine& E, const uint64_t* in_b, long in_stride, uint64_t* out, long out_stride,
-                  int npolys, int nout, cudaStream_t st);
+                  int npolys, int nout, cudaStream_t st, bool unscaled = false);
 void rescale_corrections(const Engine& E, const uint64_t* in_b, long in_stride, const uint64_t* u_l,
                          long u_stride, uint64_t* cl_tmp, long cl_stride, uint64_t* y, long y_stride, int npolys,
-                         int level, cudaStream_t st);
+                         int level, cudaStream_t st, bool unscaled = false);
 void ks_combine(const Engine& E, uint64_t* out, long out_stride, const uint64_t* base, long base_stride,
                 const uint64_t* k, long k_stride, const uint64_t* y, long y_stride, int nlimbs, int npolys,
                 int rescale_level, cudaStream_t st, int prime0 = 0);

@@ -295,12 +295,12 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
                      limb_serves(E, E.log_n, 2L * n * m, true);
   if (whole) {
     limb_tensor_inv(E, ptr, half, D2, T, n, m, st);
-    modup(E, T, half, UB, (long)kl * N, n, level, st);
+    modup(E, T, half, UB, (long)kl * N, n, level, st, true);
     KeyPtrs kp;
     for (int z = 0; z < n; z++) kp.k[z] = evk->d;
     limb_key(E, UB, KS + (long)m * N, ks, kp, n, do_rescale ? &ptr : nullptr, half, D2, U, level, st);
-    if (do_rescale) rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st);
-    else moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+    if (do_rescale) rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st, true);
+    else moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st, true);
     const int nl = do_rescale ? level : m, rl = do_rescale ? level : 0;
     bool in_place = false;                       // the two polys' clusters run apart: an operand must outlive both
     for (int z = 0; z < n; z++) in_place = in_place || out[z] == a[z] || out[z] == b[z];
@@ -326,16 +326,24 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
   } else {
     tensor_batch_op(E, ptr, half, D, n, m, st);
   }
-  if (fuse & kFuseSource) {
-    NttIo io;                                  // inverse of d2 read in place of a copy
-    io.src = D2;
-    io.src_poly_stride = k;
+  // the inverses in front of the conversions leave N^-1 to them on the NTT
+  const bool unscaled = tk == AOA_NTT;
+  NttIo inverse;
+  inverse.unscaled = true;
+  if (unscaled) {
+    NttIo io = inverse;
+    if (fuse & kFuseSource) {                  // inverse of d2 read in place of a copy
+      io.src = D2;
+      io.src_poly_stride = k;
+    } else {
+      AOA_CUDA(cudaMemcpy2DAsync(T, half * 8, D2, half * 8, (size_t)m * N * 8, n, cudaMemcpyDeviceToDevice, st));
+    }
     ntt_batch_io(E, T, n, 0, m, k, false, io, st);
   } else {
     AOA_CUDA(cudaMemcpy2DAsync(T, half * 8, D2, half * 8, (size_t)m * N * 8, n, cudaMemcpyDeviceToDevice, st));
     xform(E, tk, T, n, 0, m, k, false, st);
   }
-  modup(E, T, half, UB, (long)kl * N, n, level, st);
+  modup(E, T, half, UB, (long)kl * N, n, level, st, unscaled);
   if (tk == AOA_DGT) {
     xform(E, tk, UB, n, k, kl, kl, true, st);
     if (late) gi_keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, evk->d, KS + (long)m * N, ks, n, 0, st);
@@ -355,15 +363,16 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
     if (late) keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, evk->d, KS + (long)m * N, ks, n, 0, st);
     else keyswitch_mul_batch_op(E, D2, half, UB, (long)kl * N, evk->d, KS, ks, n, m, st);
   }
-  xform(E, tk, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
+  if (unscaled) ntt_batch_io(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, inverse, st);
+  else xform(E, tk, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
   if (late) {
     if (do_rescale) {
       if (tk == AOA_DGT) gi_hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
       else hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
       xform(E, tk, U, 2 * n, level, 1, 1, false, st);
-      rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st);
+      rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st, unscaled);
     } else {
-      moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+      moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st, unscaled);
     }
     const int nl = do_rescale ? level : m;
     xform(E, tk, Y, 2 * n, 0, nl, k, true, st);
@@ -372,7 +381,7 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
   } else if (do_rescale) {
     ks_combine(E, U, N, D + (long)level * N, half, KS + (long)level * N, ks, nullptr, 0, 1, 2 * n, 0, st, level);
     xform(E, tk, U, 2 * n, level, 1, 1, false, st);
-    rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st);
+    rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st, unscaled);
     if (fuse & kFuseCombine) {
       combine_into(C, Y, 2 * n, level, D, half, 2 * n, KS, ks, level, nullptr, 0, &outp, st);
     } else {
@@ -380,7 +389,7 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
       ks_combine_ptr(E, outp, D, half, KS, ks, Y, half, level, 2 * n, level, st);
     }
   } else {
-    moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+    moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st, unscaled);
     if (fuse & kFuseCombine) {
       combine_into(C, Y, 2 * n, m, D, half, 2 * n, KS, ks, 0, nullptr, 0, &outp, st);
     } else {
@@ -565,9 +574,9 @@ static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* co
       limb_serves(E, E.log_n, 2L * n * m, true)) {
     // small rings: whole-limb clusters (as hmult_group)
     limb_galois_inv(E, ptr, gl, half, R, T, n, m, st);
-    modup(E, T, half, UB, (long)kl * N, n, level, st);
+    modup(E, T, half, UB, (long)kl * N, n, level, st, true);
     limb_key(E, UB, KS + (long)m * N, ks, kp, n, nullptr, 0, nullptr, nullptr, level, st);
-    moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+    moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st, true);
     limb_galois_finish(E, Y, R, half, kp, outp, n, m, add, st);
     done();
     return;
@@ -576,16 +585,18 @@ static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* co
   NttIo io;                                      // inverse of the permuted c1, out of place
   io.src = X;
   io.src_poly_stride = k;
+  io.unscaled = true;                            // the conversions take N^-1 up
   ntt_batch_io(E, T, n, 0, m, k, false, io, st);
-  modup(E, T, half, UB, (long)kl * N, n, level, st);
+  modup(E, T, half, UB, (long)kl * N, n, level, st, true);
   ntt_batch(E, UB, n, k, kl, kl, true, st);
   // special limbs' key products; the Q limbs' are formed in the last pass
   if (one_key)                                   // each key word read once for the group
     keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, keys[0]->d, KS + (long)m * N, ks, n, 0, st);
   else
     keyswitch_mul_keys_op(E, nullptr, 0, UB, (long)kl * N, kp, KS + (long)m * N, ks, n, 0, st);
-  ntt_batch(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
-  moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st);
+  io.src = nullptr;
+  ntt_batch_io(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, io, st);
+  moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st, true);
   ntt_batch(E, Y, 2 * n, 0, m, k, true, st);
   galois_finish_op(E, R, half, kp, one_key, Y, outp, n, m, add, st);
   done();

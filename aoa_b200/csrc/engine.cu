@@ -139,7 +139,8 @@ static void build_rns_tables(Engine& E) {
   const int k = E.k, kl = E.kl;
   const std::vector<uint64_t>& P = E.primes;
   auto sh = [](uint64_t w, uint64_t q) { return ShoupW{w, h_shoup_companion(w, q)}; };
-  std::vector<ShoupW> modup_inv((size_t)k * k, ShoupW{0, 0});
+  std::vector<ShoupW> modup_inv((size_t)k * k, ShoupW{0, 0}), modup_inv_n = modup_inv;
+  auto by_ninv = [&](ShoupW w, uint64_t q) { return sh(h_mulmod(w.w, h_invmod((uint64_t)E.N % q, q), q), q); };
   std::vector<uint64_t> modup_hat((size_t)k * k * std::max(kl, 1), 0);
   for (int l = 0; l < k; l++) {
     for (int i = 0; i <= l; i++) {
@@ -148,6 +149,7 @@ static void build_rns_tables(Engine& E) {
       for (int t = 0; t <= l; t++)
         if (t != i) hat = h_mulmod(hat, P[t] % qi, qi);
       modup_inv[(size_t)l * k + i] = sh(h_invmod(hat, qi), qi);
+      modup_inv_n[(size_t)l * k + i] = by_ninv(modup_inv[(size_t)l * k + i], qi);
       for (int j = 0; j < kl; j++) {
         const uint64_t bj = P[k + j];
         uint64_t hb = 1;                              // (Q_l / q_i) mod b_j
@@ -157,7 +159,7 @@ static void build_rns_tables(Engine& E) {
       }
     }
   }
-  std::vector<ShoupW> moddown_inv(std::max(kl, 1), ShoupW{0, 0}), moddown_binv(k);
+  std::vector<ShoupW> moddown_inv(std::max(kl, 1), ShoupW{0, 0}), moddown_inv_n = moddown_inv, moddown_binv(k);
   std::vector<uint64_t> moddown_hat((size_t)std::max(kl, 1) * k, 0);
   for (int j = 0; j < kl; j++) {
     const uint64_t bj = P[k + j];
@@ -165,6 +167,7 @@ static void build_rns_tables(Engine& E) {
     for (int t = 0; t < kl; t++)
       if (t != j) hat = h_mulmod(hat, P[k + t] % bj, bj);
     moddown_inv[j] = sh(h_invmod(hat, bj), bj);
+    moddown_inv_n[j] = by_ninv(moddown_inv[j], bj);
     for (int i = 0; i < k; i++) {
       const uint64_t qi = P[i];
       uint64_t hq = 1;                                // (B / b_j) mod q_i
@@ -222,8 +225,10 @@ static void build_rns_tables(Engine& E) {
     E.rns.tc_moddown_binv = dev_upload(E, down_binv);
   }
   E.rns.modup_inv = dev_upload(E, modup_inv);
+  E.rns.modup_inv_n = dev_upload(E, modup_inv_n);
   E.rns.modup_hat = dev_upload(E, modup_hat);
   E.rns.moddown_inv = dev_upload(E, moddown_inv);
+  E.rns.moddown_inv_n = dev_upload(E, moddown_inv_n);
   E.rns.moddown_hat = dev_upload(E, moddown_hat);
   E.rns.moddown_binv = dev_upload(E, moddown_binv);
   E.rns.resc_inv = dev_upload(E, resc);

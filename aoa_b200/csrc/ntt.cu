@@ -99,7 +99,7 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
   if (limb_serves(E, T.log_n, (long)npolys * nlimbs, false) && (!io || io->epi.mode == kEpiStore)) {
     check_alignment(data, io);
     limb_transform(E, T, data, npolys, first_prime, nlimbs, poly_stride, forward, io ? io->src : nullptr,
-                   io ? io->src_poly_stride : 0, st);
+                   io ? io->src_poly_stride : 0, io && io->unscaled, st);
     return;
   }
   if (T.prime_kind && T.log_n >= 10) {
@@ -145,7 +145,9 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
   b.log_r = T.log_n - b.log_c;
   b.first_prime = first_prime; b.prime_shift = T.prime_shift; b.poly_stride = poly_stride;
   b.src = nullptr; b.src_poly_stride = 0; b.poly_base = 0; b.use_tma = 0;
+  b.unscaled = io && io->unscaled;
   const long n = 1L << T.log_n;
+  if (b.unscaled && (forward || T.log_n < 10)) throw AoaError(AOA_ERR_BAD_PARAM, "ntt: only inverses of N >= 2^10 leave N^-1 out");
   if (T.log_n < 10) {
     // small rings: the out-of-place source is copied first and the epilogue
     // runs as its own pass

@@ -75,6 +75,7 @@ struct Bf<kButterflyCanonical> {
     x = shoup(add_mod(U, V, q), n0, q);
     y = shoup(sub_mod(U, V, q), n1, q);
   }
+  static __device__ __forceinline__ void gs_unscaled(uint64_t& x, uint64_t& y, ShoupW w, uint64_t q) { gs(x, y, w, q, 8); }
   static __device__ __forceinline__ uint64_t fwd_out(uint64_t x, uint64_t) { return x; }
 };
 
@@ -154,6 +155,12 @@ struct Bf {
     const uint64_t b = mulw(U - V + (q << 3), n1, q);
     x = csub(csub(a, q << 1), q);
     y = csub(csub(b, q << 1), q);
+  }
+  // final inverse stage without N^-1: inputs in [0, 8q), outputs in [0, 16q)
+  static __device__ __forceinline__ void gs_unscaled(uint64_t& x, uint64_t& y, ShoupW w, uint64_t q) {
+    const uint64_t U = x, V = y;
+    x = U + V;
+    y = mulw(U - V + (q << 3), w, q);
   }
   static __device__ __forceinline__ uint64_t fwd_out(uint64_t x, uint64_t q) {   // [0, 16q + 2^32) -> [0, q)
     x = csub_hi(x, q << 3);
@@ -260,8 +267,9 @@ __device__ __forceinline__ void inv_low_s(uint64_t (&u)[Sub<LOG_S>::L], uint32_t
 }
 
 // the column pass's high digit holds the transform's final stage (half-span
-// N/2): scale by N^-1 there
-template <int LOG_S, int LAZY>
+// N/2): scale by N^-1 there, or leave the values unscaled and below 16q for a
+// basis conversion, whose first product takes N^-1 up (NttIo::unscaled)
+template <int LOG_S, int LAZY, bool UNSCALED>
 __device__ __forceinline__ void inv_high_s(uint64_t (&v)[Sub<LOG_S>::E], uint32_t itw, uint64_t q, ShoupW ninv,
                                            ShoupW ninv_w1) {
   using D = Sub<LOG_S>;
@@ -271,13 +279,19 @@ __device__ __forceinline__ void inv_high_s(uint64_t (&v)[Sub<LOG_S>::E], uint32_
 #pragma unroll
     for (int h = 0; h < D::E; h++) {
       if (h & span) continue;
-      if (i == D::HI - 1) {
-        Bf<LAZY>::gs_last(v[h], v[h + span], ninv, ninv_w1, q);
-      } else {
-        const ShoupW w = ldsw(itw + 16 * ((1 << (D::HI - 1 - i)) + (h >> (i + 1))));
-        Bf<LAZY>::gs(v[h], v[h + span], w, q, inv_bound(i, h, 8));
-      }
+      if (i == D::HI - 1) continue;
+      const ShoupW w = ldsw(itw + 16 * ((1 << (D::HI - 1 - i)) + (h >> (i + 1))));
+      Bf<LAZY>::gs(v[h], v[h + span], w, q, inv_bound(i, h, 8));
     }
+  }
+  constexpr int half = D::E / 2;
+  if constexpr (UNSCALED) {
+    const ShoupW w = ldsw(itw + 16);
+#pragma unroll
+    for (int h = 0; h < half; h++) Bf<LAZY>::gs_unscaled(v[h], v[h + half], w, q);
+  } else {
+#pragma unroll
+    for (int h = 0; h < half; h++) Bf<LAZY>::gs_last(v[h], v[h + half], ninv, ninv_w1, q);
   }
 }
 
@@ -378,6 +392,7 @@ struct NttBatch {
   long src_poly_stride;
   int poly_base;           // poly index of the launch's first poly within the call
   int spin;                // polls of a bounded wait for this kernel's own copies (engine knob)
+  bool unscaled;           // inverse column pass: without N^-1
   int use_tma;             // column pass: tiles by one tensor-map load (the kernel's tmap argument)
 };
 
@@ -422,7 +437,7 @@ struct RowTile {
 // between two buffers, so a new limb's twiddles can be written before the
 // first barrier: the buffer's previous users finished at least one item
 // earlier.
-template <int LOG_R, int DIV, int LAZY, bool FWD>
+template <int LOG_R, int DIV, int LAZY, bool FWD, bool UNSCALED = false>
 __global__ void __launch_bounds__(ColTile<LOG_R, DIV>::THREADS, ColTile<LOG_R, DIV>::MIN_BLOCKS)
 ntt_cols(NttBatch b, const __grid_constant__ CUtensorMap tmap) {
   using D = Sub<LOG_R>;
@@ -539,7 +554,7 @@ ntt_cols(NttBatch b, const __grid_constant__ CUtensorMap tmap) {
       uint64_t v[D::E];
 #pragma unroll
       for (int h = 0; h < D::E; h++) v[h] = lds64(sm + sig((h << D::LO) + t) * W * 8);
-      inv_high_s<LOG_R, LAZY>(v, stw, q, ninv, ninv_w1);
+      inv_high_s<LOG_R, LAZY, UNSCALED>(v, stw, q, ninv, ninv_w1);
 #pragma unroll
       for (int h = 0; h < D::E; h++) x[(long)((h << D::LO) + t) * C] = v[h];
     }
@@ -690,7 +705,8 @@ ntt_cols_wo(NttBatch b) {
       uint64_t v[D::E];
 #pragma unroll
       for (int h = 0; h < D::E; h++) v[h] = lds64(sm + Tl::row((h << D::LO) + t) * 8);
-      inv_high_s<LOG_R, kButterflyLazy>(v, stw, q, ninv, ninv_w1);
+      if (b.unscaled) inv_high_s<LOG_R, kButterflyLazy, true>(v, stw, q, ninv, ninv_w1);
+      else inv_high_s<LOG_R, kButterflyLazy, false>(v, stw, q, ninv, ninv_w1);
 #pragma unroll
       for (int h = 0; h < D::E; h++) x[(long)((h << D::LO) + t) * C] = v[h];
     }
@@ -922,6 +938,7 @@ static void launch_cols(const Engine& E, const NttBatch& b0, bool fwd, cudaStrea
   b.use_tma = E.tune.ntt_cols_tma && Tl::W == 16 && col_tensor_map(b, Tl::W, &map) ? 1 : 0;
   dim3 grid(C / Tl::W, ctas_per_tile(E, C / Tl::W, b.nitems, Tl::MIN_BLOCKS));
   if (fwd) launch_pdl(ntt_cols<LOG_R, DIV, LAZY, true>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
+  else if (b.unscaled) launch_pdl(ntt_cols<LOG_R, DIV, LAZY, false, true>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
   else launch_pdl(ntt_cols<LOG_R, DIV, LAZY, false>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
 }
 
@@ -1003,6 +1020,7 @@ template <int S, int DIV, int KIND>
 void allow_size() {
   allow_smem(ntt_cols<S, DIV, KIND, true>, ColTile<S, DIV>::SMEM);
   allow_smem(ntt_cols<S, DIV, KIND, false>, ColTile<S, DIV>::SMEM);
+  allow_smem(ntt_cols<S, DIV, KIND, false, true>, ColTile<S, DIV>::SMEM);
   allow_smem(ntt_rows<S, DIV, KIND, true>, RowTile<S, DIV>::SMEM);
   allow_smem(ntt_rows<S, DIV, KIND, false>, RowTile<S, DIV>::SMEM);
 }

@@ -14,6 +14,8 @@
 //
 // Modes fuse what surrounds a transform in HMult and in the automorphisms:
 //   kLimbFwd, kLimbInv    plain, in place or from a source
+//   kLimbInvUnscaled      the inverse without N^-1 (NttIo::unscaled), as in the
+//                         fused inverses whose limbs go on to a basis conversion
 //   kLimbTensorInv        d2 = a1 b1, its inverse (ModUp's input)
 //   kLimbGaloisInv        permuted c0; permuted c1 and its inverse
 //   kLimbKey              forward of a ModUp limb, key product, inverse: one
@@ -42,7 +44,9 @@ struct Limb {
   static_assert(LR % 2 == 0 && W >= 4, "column rounds are radix 4");
 };
 
-enum { kLimbFwd, kLimbInv, kLimbTensorInv, kLimbGaloisInv, kLimbKey, kLimbFinish, kLimbGaloisFinish };
+enum {
+  kLimbFwd, kLimbInv, kLimbInvUnscaled, kLimbTensorInv, kLimbGaloisInv, kLimbKey, kLimbFinish, kLimbGaloisFinish
+};
 constexpr bool limb_has_fwd(int mode) { return mode == kLimbFwd || mode >= kLimbKey; }
 constexpr bool limb_has_inv(int mode) { return mode >= kLimbInv && mode <= kLimbKey; }
 
@@ -219,7 +223,7 @@ __device__ __forceinline__ void limb_fwd(const LimbSmem& s, uint32_t rank, uint6
 // x.  WAIT: the barrier that every CTA of the cluster arrives at when it starts
 // is still to be waited for (a forward transform has done so, and its own
 // barrier has every column tile read).
-template <class L, int KIND, bool WAIT>
+template <class L, int KIND, bool WAIT, bool UNSCALED>
 __device__ __forceinline__ void limb_inv(const LimbSmem& s, uint32_t rank, uint64_t* x, const PrimeConst& P) {
   const int tid = threadIdx.x;
   const uint64_t q = P.q;
@@ -288,9 +292,15 @@ __device__ __forceinline__ void limb_inv(const LimbSmem& s, uint32_t rank, uint6
         Bf<KIND>::gs(v[1], v[3], w0, q, 8);
 #pragma unroll
         for (int j = 0; j < 4; j++) sts64(a + j * step, v[j]);
-      } else {                             // the last stage, with N^-1
-        Bf<KIND>::gs_last(v[0], v[2], ninv, ninv_w1, q);
-        Bf<KIND>::gs_last(v[1], v[3], ninv, ninv_w1, q);
+      } else {                             // the last stage, with N^-1 or left unscaled
+        if constexpr (UNSCALED) {
+          const ShoupW w0 = ldsw(s.ti + 16);
+          Bf<KIND>::gs_unscaled(v[0], v[2], w0, q);
+          Bf<KIND>::gs_unscaled(v[1], v[3], w0, q);
+        } else {
+          Bf<KIND>::gs_last(v[0], v[2], ninv, ninv_w1, q);
+          Bf<KIND>::gs_last(v[1], v[3], ninv, ninv_w1, q);
+        }
         uint64_t* o = x + rank * L::W + w;
 #pragma unroll
         for (int j = 0; j < 4; j++) o[(long)(r0 + j * d) * L::C] = v[j];
@@ -330,7 +340,7 @@ __device__ __forceinline__ void limb_run(const LimbArgs& a, const typename EndsO
                               : ks_sum2(A[i], B[i], D[i], k, fit, P));
       }
       __syncthreads();
-      limb_inv<L, KIND, true>(s, rank, e.U + (long)p * L::N, P);
+      limb_inv<L, KIND, true, false>(s, rank, e.U + (long)p * L::N, P);
       return;
     }
     limb_fwd<L, KIND>(s, rank, q);
@@ -339,7 +349,7 @@ __device__ __forceinline__ void limb_run(const LimbArgs& a, const typename EndsO
     for (int i = tid; i < L::M; i += L::P)
       sts64(word(i), mul_mod(Bf<KIND>::fwd_out(lds64(word(i)), q), key[i], P));
     __syncthreads();
-    limb_inv<L, KIND, false>(s, rank, x, P);
+    limb_inv<L, KIND, false, true>(s, rank, x, P);
   } else if constexpr (MODE == kLimbFwd) {
     limb_fwd<L, KIND>(s, rank, q);
 #pragma unroll 2
@@ -374,7 +384,7 @@ __device__ __forceinline__ void limb_run(const LimbArgs& a, const typename EndsO
       out[i] = e.add ? add_mod(out[i], c, q) : c;
     }
   } else {
-    if constexpr (MODE == kLimbInv) {
+    if constexpr (MODE == kLimbInv || MODE == kLimbInvUnscaled) {
       const uint64_t* src = (a.src ? a.src + (long)p * a.src_poly_stride * L::N + limb_off : x) + row0;
 #pragma unroll 4
       for (int i = tid; i < L::M; i += L::P) sts64(word(i), src[i]);
@@ -405,7 +415,7 @@ __device__ __forceinline__ void limb_run(const LimbArgs& a, const typename EndsO
       x = a.data + (long)z * a.poly_stride * L::N + limb_off;
     }
     __syncthreads();
-    limb_inv<L, KIND, true>(s, rank, x, P);
+    limb_inv<L, KIND, true, MODE != kLimbInv>(s, rank, x, P);
   }
 }
 
@@ -524,6 +534,7 @@ template <class L>
 void limb_allow_all() {
   limb_allow<L, kLimbFwd>();
   limb_allow<L, kLimbInv>();
+  limb_allow<L, kLimbInvUnscaled>();
   limb_allow<L, kLimbTensorInv>();
   limb_allow<L, kLimbGaloisInv>();
   limb_allow<L, kLimbKey>();
@@ -570,7 +581,8 @@ bool limb_serves(const Engine& E, int log_n, long items, bool fused) {
 }
 
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
-                    long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, cudaStream_t st) {
+                    long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, bool unscaled,
+                    cudaStream_t st) {
   LimbArgs a = limb_args(E);
   a.tw = T.tw;
   a.itw = T.itw;
@@ -583,6 +595,7 @@ void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npo
   a.first_prime = first_prime;
   a.prime_shift = T.prime_shift;
   if (forward) limb_dispatch<kLimbFwd>(T.log_n, a, NoEnds{}, nlimbs, st);
+  else if (unscaled) limb_dispatch<kLimbInvUnscaled>(T.log_n, a, NoEnds{}, nlimbs, st);
   else limb_dispatch<kLimbInv>(T.log_n, a, NoEnds{}, nlimbs, st);
 }
 

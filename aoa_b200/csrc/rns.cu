@@ -529,7 +529,7 @@ void rns_init(Engine& E) {
 
 // ModUp: Q limbs 0..level of `in` (coefficient domain) -> kl B limbs of `out_b`.
 void modup(const Engine& E, const uint64_t* in, long in_stride, uint64_t* out_b, long out_stride,
-           int npolys, int level, cudaStream_t st) {
+           int npolys, int level, cudaStream_t st, bool unscaled) {
   if (E.kl == 0) return;
   if (level < 0 || level >= E.k) throw AoaError(AOA_ERR_BAD_PARAM, "modup: bad level");
   ConvArgs a{};
@@ -537,20 +537,21 @@ void modup(const Engine& E, const uint64_t* in, long in_stride, uint64_t* out_b,
   a.in_poly_stride = in_stride; a.out_poly_stride = out_stride;
   a.nin = level + 1; a.mat_ld = E.kl;
   a.in_prime0 = 0; a.out_prime0 = E.k;
-  a.zc = E.rns.modup_inv + (long)level * E.k;
+  a.zc = (unscaled ? E.rns.modup_inv_n : E.rns.modup_inv) + (long)level * E.k;
   a.mat = E.rns.modup_hat + (long)level * E.k * E.kl;
   a.tc_b = E.rns.tc_modup ? E.rns.tc_modup + (size_t)level * kTcB : nullptr;
   a.pc = E.d_pc; a.log_n = E.log_n; a.mode = kRaw;
   run_convert(E, a, npolys, 0, E.kl, st);
 }
 
-static ConvArgs moddown_args(const Engine& E, const uint64_t* in_b, long in_stride, uint64_t* out, long out_stride) {
+static ConvArgs moddown_args(const Engine& E, const uint64_t* in_b, long in_stride, uint64_t* out, long out_stride,
+                             bool unscaled) {
   ConvArgs a{};
   a.in = in_b; a.out = out;
   a.in_poly_stride = in_stride; a.out_poly_stride = out_stride;
   a.nin = E.kl; a.mat_ld = E.k;
   a.in_prime0 = E.k; a.out_prime0 = 0;
-  a.zc = E.rns.moddown_inv;
+  a.zc = unscaled ? E.rns.moddown_inv_n : E.rns.moddown_inv;
   a.mat = E.rns.moddown_hat;
   a.tc_b = E.rns.tc_moddown;
   a.binv = E.rns.moddown_binv; a.pc = E.d_pc; a.log_n = E.log_n;
@@ -562,15 +563,15 @@ static ConvArgs moddown_args(const Engine& E, const uint64_t* in_b, long in_stri
 void moddown(const Engine& E, const uint64_t* in_q, const uint64_t* in_b, long in_stride, uint64_t* out,
              long out_stride, int npolys, int level, cudaStream_t st) {
   if (level < 0 || level >= E.k) throw AoaError(AOA_ERR_BAD_PARAM, "moddown: bad level");
-  ConvArgs a = moddown_args(E, in_b, in_stride, out, out_stride);
+  ConvArgs a = moddown_args(E, in_b, in_stride, out, out_stride, false);
   a.x = in_q; a.x_poly_stride = in_stride; a.mode = kModDown;
   run_convert(E, a, npolys, 0, level + 1, st);
 }
 
 // conv_i (coefficient domain) of ModDown for outputs 0..nout-1, written to out.
 void moddown_conv(const Engine& E, const uint64_t* in_b, long in_stride, uint64_t* out, long out_stride,
-                  int npolys, int nout, cudaStream_t st) {
-  ConvArgs a = moddown_args(E, in_b, in_stride, out, out_stride);
+                  int npolys, int nout, cudaStream_t st, bool unscaled) {
+  ConvArgs a = moddown_args(E, in_b, in_stride, out, out_stride, unscaled);
   a.mode = kRaw;
   run_convert(E, a, npolys, 0, nout, st);
 }
@@ -581,8 +582,8 @@ void moddown_conv(const Engine& E, const uint64_t* in_b, long in_stride, uint64_
 // One launch when level < 32, else c_l first (into cl_tmp) and then the y_i.
 void rescale_corrections(const Engine& E, const uint64_t* in_b, long in_stride, const uint64_t* u_l,
                          long u_stride, uint64_t* cl_tmp, long cl_stride, uint64_t* y, long y_stride, int npolys,
-                         int level, cudaStream_t st) {
-  ConvArgs a = moddown_args(E, in_b, in_stride, y, y_stride);
+                         int level, cudaStream_t st, bool unscaled) {
+  ConvArgs a = moddown_args(E, in_b, in_stride, y, y_stride, unscaled);
   a.tc_b = E.rns.tc_moddown_binv;                // the tensor-core kernel's rescale modes fold B^-1 in
   if (level < kConvOut) {
     a.mode = kRescaleFused;
@@ -590,7 +591,7 @@ void rescale_corrections(const Engine& E, const uint64_t* in_b, long in_stride, 
     run_convert(E, a, npolys, 0, level + 1, st);
     return;
   }
-  ConvArgs t = moddown_args(E, in_b, in_stride, cl_tmp, cl_stride);
+  ConvArgs t = moddown_args(E, in_b, in_stride, cl_tmp, cl_stride, unscaled);
   t.tc_b = E.rns.tc_moddown_binv;
   t.mode = kRescaleTop;
   t.d = u_l; t.d_poly_stride = u_stride;

@@ -1,0 +1,55 @@
+"""HMult and rotations whose inverse transforms leave N^-1 to the basis conversions:
+both conversion kernels, every fusing mode, transforms of one call on whole-limb
+and two-pass kernels at once, all-(q - 1) operands, against the oracle."""
+import numpy as np
+import pytest
+
+from oracle import ST_NTT, Oracle
+from tests.ckks_inputs import make_keys, uniform_residues
+from tests.gpu_util import require_gpu
+
+pytestmark = pytest.mark.gpu
+SCALE = 1 << 40
+
+
+def _primes(bits, log_n, count):
+    from aoa_b200 import params
+    if bits == "q1":
+        return params.ntt_primes(60, 1 << 32, count)
+    if bits == "mixed":
+        return params.ntt_primes(63, 2 << log_n, 1) + params.ntt_primes(55, 2 << log_n, count - 1)
+    return params.ntt_primes(bits, 2 << log_n, count)
+
+
+# 4 limbs of 2^15 are whole-limb transforms, the 22 key-product limbs two passes
+@pytest.mark.parametrize("log_n,k,kl", [(12, 3, 4), (15, 4, 11)])
+@pytest.mark.parametrize("bits", ["q1", "mixed", 60, 62, 34])
+@pytest.mark.parametrize("fuse,tensor_cores", [(1, 1), (1, 0), (0, 1), (7, 1)])
+def test_hmult_and_rotation(log_n, k, kl, bits, fuse, tensor_cores):
+    require_gpu()
+    import aoa_b200 as aoa
+    ps = _primes(bits, log_n, k + kl)
+    E = aoa.Engine(log_n, ps[:k], ps[k:])
+    E.tune("fuse", fuse)
+    E.tune("conv_tensor_cores", tensor_cores)
+    ctx, o = aoa.Context(E), Oracle(E.N, ps[:k], ps[k:])
+    keys = make_keys(o, seed=3, rotations=(5,))
+    rng = np.random.default_rng(k)
+    top = np.repeat(np.array(ps[:k], dtype=np.uint64)[:, None] - np.uint64(1), E.N, axis=1)
+    host = [(top, top), (uniform_residues(rng, ps[:k], E.N), uniform_residues(rng, ps[:k], E.N))]
+    a, b = [aoa.Ciphertext.from_residues(ctx, *h, slots=8, scale=SCALE, domain=aoa.AOA_NTT) for h in host]
+    out = aoa.Ciphertext(ctx)
+    aoa.ckks_mul(ctx, out, a, b, aoa.SwitchKey(ctx, *keys["evk"]))
+    w0, w1, _ = o.hmult(host[0], host[1], keys["evk"], k - 1, SCALE, SCALE, rescale=True, a_state=ST_NTT,
+                        b_state=ST_NTT)
+    g0, g1 = out.download(nlimbs=k - 1, domain=aoa.AOA_COEF)
+    assert np.array_equal(g0, w0[: k - 1]) and np.array_equal(g1, w1[: k - 1])
+    E2 = aoa.Engine(log_n, ps[:k], ps[k:])       # rotations: against the reference's op sequence
+    ctx2 = aoa.Context(E2)
+    for c in host:
+        got, want = aoa.Ciphertext(ctx), aoa.Ciphertext(ctx2)
+        x, y = [aoa.Ciphertext.from_residues(t, *c, slots=8, scale=SCALE, domain=aoa.AOA_NTT) for t in (ctx, ctx2)]
+        aoa.ckks_rotate_left(ctx, got, x, 5, aoa.SwitchKey(ctx, *keys["rtk"][5]))
+        aoa.ckks_rotate_plain(ctx2, want, y, 5, aoa.SwitchKey(ctx2, *keys["rtk"][5]))
+        for u, v in zip(got.download(nlimbs=k, domain=aoa.AOA_COEF), want.download(nlimbs=k, domain=aoa.AOA_COEF)):
+            assert np.array_equal(u, v)
