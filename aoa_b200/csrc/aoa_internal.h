@@ -291,6 +291,7 @@ struct NttIo {
   const uint64_t* src = nullptr;
   long src_poly_stride = 0;
   bool unscaled = false;
+  int prime_gap = 0;       // limbs after the first are under primes this much further on
   NttEpi epi;
 };
 void ntt_init(Engine& E);
@@ -307,8 +308,7 @@ void ntt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int
 void limb_init(const Engine& E);
 bool limb_serves(const Engine& E, int log_n, long items, bool fused);
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
-                    long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, bool unscaled,
-                    cudaStream_t st);
+                    long poly_stride, bool forward, const NttIo& io, cudaStream_t st);
 // D2 + z half = a1 b1 and T + z half = its unscaled inverse transform, op z
 void limb_tensor_inv(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, uint64_t* T, int n, int nlimbs,
                      cudaStream_t st);
@@ -337,7 +337,7 @@ void moddown_conv(const Engine& E, const uint64_t* in_b, long in_stride, uint64_
                   int npolys, int nout, cudaStream_t st, bool unscaled = false);
 void rescale_corrections(const Engine& E, const uint64_t* in_b, long in_stride, const uint64_t* u_l,
                          long u_stride, uint64_t* cl_tmp, long cl_stride, uint64_t* y, long y_stride, int npolys,
-                         int level, cudaStream_t st, bool unscaled = false);
+                         int level, cudaStream_t st, bool unscaled = false, bool top_unscaled = false);
 void ks_combine(const Engine& E, uint64_t* out, long out_stride, const uint64_t* base, long base_stride,
                 const uint64_t* k, long k_stride, const uint64_t* y, long y_stride, int nlimbs, int npolys,
                 int rescale_level, cudaStream_t st, int prime0 = 0);
@@ -382,7 +382,7 @@ void ks_combine_ptr(const Engine& E, const OutPtrs& outp, const uint64_t* base, 
 // ks_finish.cu: the Q limbs of a key switch in one pass over the operands
 void tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, int n, int nlimbs, cudaStream_t st);
 void hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key, uint64_t* U,
-                  int n, int level, cudaStream_t st);
+                  long u_stride, int n, int level, cudaStream_t st);
 void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,
                      const uint64_t* Y, const OutPtrs& outp, int n, int nlimbs, int rescale_level, cudaStream_t st);
 // the same with Gaussian-integer products (DGT domain, planar limbs)

@@ -363,12 +363,28 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
     if (late) keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, evk->d, KS + (long)m * N, ks, n, 0, st);
     else keyswitch_mul_batch_op(E, D2, half, UB, (long)kl * N, evk->d, KS, ks, n, m, st);
   }
-  if (unscaled) ntt_batch_io(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, inverse, st);
-  else xform(E, tk, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
+  // the top Q limb of d + d2 key B^-1 takes the free place before the special
+  // limbs and runs in their inverse, unless its 2 n limbs alone are more than one
+  // wave of the transform's CTAs (tiles of 4096 words, three to an SM).  Measured
+  // (us, alone -> joined): one HMult at 2^16 301.3 -> 293.7, 24 of mixed levels at
+  // 2^15 2678 -> 2533; 24 to a launch at 2^16 (1.7 waves) 9222 -> 9253.
+  const bool joined = late && do_rescale && tk == AOA_NTT && 2L * n * N <= 3L * E.num_sms * 4096;
+  uint64_t* top = KS + (long)level * N;
+  if (joined) {
+    hmult_top_op(E, ptr, half, D2, evk->d, top, ks, n, level, st);
+    inverse.prime_gap = k - m;
+    ntt_batch_io(E, top, 2 * n, level, kl + 1, k + kl, false, inverse, st);
+  } else if (unscaled) {
+    ntt_batch_io(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, inverse, st);
+  } else {
+    xform(E, tk, KS + (long)m * N, 2 * n, k, kl, k + kl, false, st);
+  }
   if (late) {
-    if (do_rescale) {
+    if (joined) {
+      rescale_corrections(E, KS + (long)m * N, ks, top, ks, CL, N, Y, half, 2 * n, level, st, true, true);
+    } else if (do_rescale) {
       if (tk == AOA_DGT) gi_hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
-      else hmult_top_op(E, ptr, half, D2, evk->d, U, n, level, st);
+      else hmult_top_op(E, ptr, half, D2, evk->d, U, N, n, level, st);
       xform(E, tk, U, 2 * n, level, 1, 1, false, st);
       rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st, unscaled);
     } else {

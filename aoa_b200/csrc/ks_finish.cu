@@ -38,10 +38,10 @@ __global__ void __launch_bounds__(kThreads) tensor_d2(const __grid_constant__ Ct
 }
 
 // Limb `level` of d + ModDown's Q part (no correction): U[poly][z] = limb
-// `level` of (a0 b0 + d2 kb B^-1, a0 b1 + a1 b0 + d2 ka B^-1)
+// `level` of (a0 b0 + d2 kb B^-1, a0 b1 + a1 b0 + d2 ka B^-1), polys u_stride apart
 __global__ void __launch_bounds__(kThreads) hmult_top(const __grid_constant__ CtPtrs ptr, long half,
                                                       const uint64_t* D2, const uint64_t* key, long key_half,
-                                                      uint64_t* U, int n, int level, const ShoupW* binv,
+                                                      uint64_t* U, long u_stride, int n, int level, const ShoupW* binv,
                                                       const PrimeConst* pc, int log_n) {
   pdl_begin();
   const long N = 1L << log_n;
@@ -53,8 +53,8 @@ __global__ void __launch_bounds__(kThreads) hmult_top(const __grid_constant__ Ct
   const uint64_t kb = shoup(key[off], bi, P.q), ka = shoup(key[key_half + off], bi, P.q);
   const uint64_t *a = ptr.a[z] + off, *b = ptr.b[z] + off;
   const uint64_t a0 = a[0], a1 = a[half], b0 = b[0], b1 = b[half], d2 = D2[(long)z * half + off];
-  U[(long)z * N + c] = ks_sum2(a0, b0, d2, kb, fit, P);
-  U[(long)(n + z) * N + c] = ks_sum3(a0, a1, b0, b1, d2, ka, fit, P);
+  U[z * u_stride + c] = ks_sum2(a0, b0, d2, kb, fit, P);
+  U[(n + z) * u_stride + c] = ks_sum3(a0, a1, b0, b1, d2, ka, fit, P);
 }
 
 // out = (d + d2 key B^-1 - y) q_l^-1 (RESC, y = the merged ModDown + rescale
@@ -256,9 +256,9 @@ void tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, i
 }
 
 void hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key, uint64_t* U,
-                  int n, int level, cudaStream_t st) {
-  launch_pdl(hmult_top, dim3(E.N / kThreads, 1, n), kThreads, 0, st, ptr, half, D2, key, (long)E.nprimes * E.N, U, n,
-             level, E.rns.moddown_binv, E.d_pc, E.log_n);
+                  long u_stride, int n, int level, cudaStream_t st) {
+  launch_pdl(hmult_top, dim3(E.N / kThreads, 1, n), kThreads, 0, st, ptr, half, D2, key, (long)E.nprimes * E.N, U,
+             u_stride, n, level, E.rns.moddown_binv, E.d_pc, E.log_n);
 }
 
 void hmult_finish_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key,

@@ -44,7 +44,7 @@ __global__ void ntt_small(NttBatch b, bool fwd) {
   const int N = 1 << b.log_n;
   for (int j = blockIdx.x; j < b.nitems; j += gridDim.x) {
     const int limb = j / b.npolys, p = j % b.npolys;
-    const int prime = b.first_prime + (limb >> b.prime_shift);
+    const int prime = b.prime_of(limb);
     uint64_t* x = b.data + ((long)p * b.poly_stride + limb) * N;
     const PrimeConst& P = b.pc[prime];
     const uint64_t q = P.q;
@@ -94,12 +94,12 @@ static void check_alignment(const uint64_t* data, const NttIo* io) {
 void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
                       long poly_stride, bool forward, cudaStream_t st, const NttIo* io) {
   if (npolys <= 0 || nlimbs <= 0) return;
-  if (first_prime < 0 || first_prime + ((nlimbs - 1) >> T.prime_shift) >= E.nprimes)
+  const int gap = io && nlimbs > 1 ? io->prime_gap : 0;
+  if (first_prime < 0 || first_prime + ((nlimbs - 1) >> T.prime_shift) + gap >= E.nprimes)
     throw AoaError(AOA_ERR_BAD_PARAM, "ntt: prime range out of bounds");
   if (limb_serves(E, T.log_n, (long)npolys * nlimbs, false) && (!io || io->epi.mode == kEpiStore)) {
     check_alignment(data, io);
-    limb_transform(E, T, data, npolys, first_prime, nlimbs, poly_stride, forward, io ? io->src : nullptr,
-                   io ? io->src_poly_stride : 0, io && io->unscaled, st);
+    limb_transform(E, T, data, npolys, first_prime, nlimbs, poly_stride, forward, io ? *io : NttIo{}, st);
     return;
   }
   if (T.prime_kind && T.log_n >= 10) {
@@ -110,7 +110,7 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
     // rest.  Runs start at prime boundaries; each run's data, source and
     // epilogue limbs are offset by its first limb.
     const long n = 1L << T.log_n;
-    auto kind_at = [&](int l) { return (int)T.prime_kind[first_prime + (l >> T.prime_shift)]; };
+    auto kind_at = [&](int l) { return (int)T.prime_kind[first_prime + (l >> T.prime_shift) + (l ? gap : 0)]; };
     for (int l0 = 0; l0 < nlimbs;) {
       const int kind = kind_at(l0);
       int l1 = l0 + 1;
@@ -126,8 +126,9 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
       if (io) run = *io;
       if (run.src) run.src += (long)l0 * n;
       run.epi.limb_base += l0;
-      ntt_batch_tables(E, T2, data + (long)l0 * n, npolys, first_prime + (l0 >> T.prime_shift), l1 - l0,
-                       poly_stride, forward, st, &run);
+      if (l0) run.prime_gap = 0;                 // it is in the run's first prime
+      ntt_batch_tables(E, T2, data + (long)l0 * n, npolys, first_prime + (l0 >> T.prime_shift) + (l0 ? gap : 0),
+                       l1 - l0, poly_stride, forward, st, &run);
       l0 = l1;
     }
     return;
@@ -146,8 +147,10 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
   b.first_prime = first_prime; b.prime_shift = T.prime_shift; b.poly_stride = poly_stride;
   b.src = nullptr; b.src_poly_stride = 0; b.poly_base = 0; b.use_tma = 0;
   b.unscaled = io && io->unscaled;
+  b.prime_gap = gap;
   const long n = 1L << T.log_n;
-  if (b.unscaled && (forward || T.log_n < 10)) throw AoaError(AOA_ERR_BAD_PARAM, "ntt: only inverses of N >= 2^10 leave N^-1 out");
+  if ((b.unscaled && forward) || ((b.unscaled || gap) && T.log_n < 10))
+    throw AoaError(AOA_ERR_BAD_PARAM, "ntt: only inverses of N >= 2^10 leave N^-1 out");
   if (T.log_n < 10) {
     // small rings: the out-of-place source is copied first and the epilogue
     // runs as its own pass

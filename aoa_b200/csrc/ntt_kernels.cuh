@@ -385,7 +385,8 @@ struct NttBatch {
   unsigned* err;           // device error word
   int log_n, log_r, log_c; // N = R * C
   int first_prime;
-  int prime_shift;         // limb l uses prime first_prime + (l >> prime_shift)
+  int prime_shift;         // limb l uses prime first_prime + (l >> prime_shift) ...
+  int prime_gap;           // ... + prime_gap for l > 0
   long poly_stride;        // limbs between consecutive polys
   int npolys, nitems;      // nitems = nlimbs * npolys
   const uint64_t* src;     // this pass loads from src (out of place) when set
@@ -394,6 +395,9 @@ struct NttBatch {
   int spin;                // polls of a bounded wait for this kernel's own copies (engine knob)
   bool unscaled;           // inverse column pass: without N^-1
   int use_tma;             // column pass: tiles by one tensor-map load (the kernel's tmap argument)
+  __device__ __forceinline__ int prime_of(int limb) const {
+    return first_prime + (limb >> prime_shift) + (limb ? prime_gap : 0);
+  }
 };
 
 // Threads per SM the pass kernels are compiled for (register budget).
@@ -494,7 +498,7 @@ ntt_cols(NttBatch b, const __grid_constant__ CUtensorMap tmap) {
   auto twiddles = [&](int limb) {          // the other buffer's users are at least one item behind
     if (limb == cur_limb) return;
     tb ^= 1;
-    const ShoupW* tw = (FWD ? b.tw : b.itw) + (long)(b.first_prime + (limb >> b.prime_shift)) * N;
+    const ShoupW* tw = (FWD ? b.tw : b.itw) + (long)b.prime_of(limb) * N;
     for (int e = threadIdx.x; e < D::S; e += blockDim.x) tws[tb * D::S + e] = tw[e];
     cur_limb = limb;
   };
@@ -503,7 +507,7 @@ ntt_cols(NttBatch b, const __grid_constant__ CUtensorMap tmap) {
   if (j_lo < j_hi) issue(j_lo, 0);
   for (int j = j_lo, it = 0; j < j_hi; j++, it++) {
     const int bi = it & 1;
-    const int limb = j / b.npolys, prime = b.first_prime + (limb >> b.prime_shift);
+    const int limb = j / b.npolys, prime = b.prime_of(limb);
     twiddles(limb);
     const bool ok = mbar_wait(&mbar[bi], (it >> 1) & 1, b.spin);
     if (__syncthreads_or(!ok)) {
@@ -618,7 +622,7 @@ ntt_cols_wo(NttBatch b) {
   }
   __syncthreads();
   const int j_lo = (int)((long)blockIdx.y * b.nitems / G), j_hi = (int)((long)(blockIdx.y + 1) * b.nitems / G);
-  auto prime_of = [&](int j) { return b.first_prime + ((j / b.npolys) >> b.prime_shift); };
+  auto prime_of = [&](int j) { return b.prime_of(j / b.npolys); };
   pdl_begin();
   if (warp == NW) {
     // producer: tile rows of W words (one bulk copy each) and, when the prime
@@ -772,7 +776,7 @@ ntt_rows(NttBatch b, const __grid_constant__ NttEpi epi) {
   auto twiddles = [&](int limb) {          // the other buffer's users are at least one item behind
     if (limb == cur_limb) return;
     tb ^= 1;
-    const int prime = b.first_prime + (limb >> b.prime_shift);
+    const int prime = b.prime_of(limb);
     const ShoupW* tw = (FWD ? b.tw : b.itw) + (long)prime * N;
     for (int e = threadIdx.x; e < ROWS * NT1; e += blockDim.x) {
       const int r = e / NT1, jj = e % NT1;
@@ -837,7 +841,7 @@ ntt_rows(NttBatch b, const __grid_constant__ NttEpi epi) {
       } else {
         const int limb = j / b.npolys;
         const long p = b.poly_base + j % b.npolys;
-        const int prime = b.first_prime + (limb >> b.prime_shift);
+        const int prime = b.prime_of(limb);
         const PrimeConst& P = b.pc[prime];
         const long c0 = (long)(row0 + rho) << LOG_C;
 #pragma unroll

@@ -58,7 +58,7 @@ struct LimbArgs {
   const ShoupW *tw, *itw;
   const PrimeConst* pc;
   unsigned* err;
-  int npolys, first_prime, prime_shift, spin;
+  int npolys, first_prime, prime_shift, prime_gap, spin;   // primes of the limbs as in NttBatch
 };
 
 struct NoEnds {};
@@ -428,7 +428,7 @@ limb_kernel(const __grid_constant__ LimbArgs a, const __grid_constant__ typename
   const int tid = threadIdx.x;
   const uint32_t rank = blockIdx.x % L::CL;
   const int item = blockIdx.x / L::CL, limb = item / a.npolys, p = item % a.npolys;
-  int prime = a.first_prime + (limb >> a.prime_shift);
+  int prime = a.first_prime + (limb >> a.prime_shift) + (limb ? a.prime_gap : 0);
   bool fwd = FWD;
   if constexpr (MODE == kLimbKey)
     if (limb == e.kl) {                    // the top Q limb: inverse only
@@ -581,21 +581,21 @@ bool limb_serves(const Engine& E, int log_n, long items, bool fused) {
 }
 
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
-                    long poly_stride, bool forward, const uint64_t* src, long src_poly_stride, bool unscaled,
-                    cudaStream_t st) {
+                    long poly_stride, bool forward, const NttIo& io, cudaStream_t st) {
   LimbArgs a = limb_args(E);
   a.tw = T.tw;
   a.itw = T.itw;
   a.pc = T.pc;
   a.data = data;
   a.poly_stride = poly_stride;
-  a.src = src;
-  a.src_poly_stride = src_poly_stride;
+  a.src = io.src;
+  a.src_poly_stride = io.src_poly_stride;
+  a.prime_gap = io.prime_gap;
   a.npolys = npolys;
   a.first_prime = first_prime;
   a.prime_shift = T.prime_shift;
   if (forward) limb_dispatch<kLimbFwd>(T.log_n, a, NoEnds{}, nlimbs, st);
-  else if (unscaled) limb_dispatch<kLimbInvUnscaled>(T.log_n, a, NoEnds{}, nlimbs, st);
+  else if (io.unscaled) limb_dispatch<kLimbInvUnscaled>(T.log_n, a, NoEnds{}, nlimbs, st);
   else limb_dispatch<kLimbInv>(T.log_n, a, NoEnds{}, nlimbs, st);
 }
 

@@ -58,6 +58,7 @@ struct ConvArgs {
   const uint8_t* tc_b;      // tensor-core image of `mat` (null: CUDA-core kernel only)
   unsigned* err;            // device error word
   int npolys;
+  bool d_unscaled;          // u_l lacks N^-1 and is any word congruent to it
   int spin;                 // polls of a bounded wait for this kernel's own copies and MMAs (engine knob)
 };
 
@@ -106,6 +107,10 @@ basis_convert(ConvArgs a, int j_first, int j_end) {
   uint64_t* out = a.out + blockIdx.y * a.out_poly_stride + c;
   uint64_t dv = 0;
   if (a.mode >= kRescaleTop) dv = a.d[blockIdx.y * a.d_poly_stride + c];
+  if (a.d_unscaled) {                                    // prime of the last output
+    const PrimeConst& P = a.pc[a.out_prime0 + j_end - 1];
+    dv = shoup(dv, P.ninv, P.ninv_sh, P.q);
+  }
   if (a.mode == kRescaleFused) {
     // outputs 0..l with l = j_end - 1 < kConvOut: c_l first, shared through smem
     __shared__ uint64_t s_cl[kConvCoefs];
@@ -412,7 +417,11 @@ basis_convert_tc(ConvArgs a, int j_first, int j_end) {
     const long c = c0 + g * 32 + lane;
     const uint32_t t_lane = tmem + ((uint32_t)(g * 32) << 16);
     uint64_t* out = a.out + poly * a.out_poly_stride + c;
-    const uint64_t dv = dv_cur;
+    uint64_t dv = dv_cur;
+    if ((MODE == kRescaleTop || MODE == kRescaleFused) && a.d_unscaled) {   // under the last output's prime
+      const PrimeConst* Pl = a.pc + a.out_prime0 + j_end - 1;
+      dv = tc_scale<Q1>(dv, ShoupW{Pl->ninv, Pl->ninv_sh}, s_out[j_end - 1].q);
+    }
     uint32_t v[16];
     if (MODE == kRescaleFused) {
       const int l = j_end - 1;                 // outputs 0..l-1 from c_l (j_first = 0)
@@ -582,19 +591,19 @@ void moddown_conv(const Engine& E, const uint64_t* in_b, long in_stride, uint64_
 // One launch when level < 32, else c_l first (into cl_tmp) and then the y_i.
 void rescale_corrections(const Engine& E, const uint64_t* in_b, long in_stride, const uint64_t* u_l,
                          long u_stride, uint64_t* cl_tmp, long cl_stride, uint64_t* y, long y_stride, int npolys,
-                         int level, cudaStream_t st, bool unscaled) {
+                         int level, cudaStream_t st, bool unscaled, bool top_unscaled) {
   ConvArgs a = moddown_args(E, in_b, in_stride, y, y_stride, unscaled);
   a.tc_b = E.rns.tc_moddown_binv;                // the tensor-core kernel's rescale modes fold B^-1 in
   if (level < kConvOut) {
     a.mode = kRescaleFused;
-    a.d = u_l; a.d_poly_stride = u_stride;
+    a.d = u_l; a.d_poly_stride = u_stride; a.d_unscaled = top_unscaled;
     run_convert(E, a, npolys, 0, level + 1, st);
     return;
   }
   ConvArgs t = moddown_args(E, in_b, in_stride, cl_tmp, cl_stride, unscaled);
   t.tc_b = E.rns.tc_moddown_binv;
   t.mode = kRescaleTop;
-  t.d = u_l; t.d_poly_stride = u_stride;
+  t.d = u_l; t.d_poly_stride = u_stride; t.d_unscaled = top_unscaled;
   t.out_shift = level;
   run_convert(E, t, npolys, level, level + 1, st);
   a.mode = kRescaleY;

@@ -1,6 +1,7 @@
 """HMult and rotations whose inverse transforms leave N^-1 to the basis conversions:
 both conversion kernels, every fusing mode, transforms of one call on whole-limb
-and two-pass kernels at once, all-(q - 1) operands, against the oracle."""
+and two-pass kernels at once, all-(q - 1) operands, against the oracle; and the
+rescaled limb inside and outside the special limbs' inverse."""
 import numpy as np
 import pytest
 
@@ -53,3 +54,31 @@ def test_hmult_and_rotation(log_n, k, kl, bits, fuse, tensor_cores):
         aoa.ckks_rotate_plain(ctx2, want, y, 5, aoa.SwitchKey(ctx2, *keys["rtk"][5]))
         for u, v in zip(got.download(nlimbs=k, domain=aoa.AOA_COEF), want.download(nlimbs=k, domain=aoa.AOA_COEF)):
             assert np.array_equal(u, v)
+
+
+@pytest.mark.parametrize("n", [55, 56])
+@pytest.mark.parametrize("m", [2, 4])
+def test_rescaled_limb_joins_the_special_limbs_up_to_one_wave(n, m):
+    """Batches at 2^14 on both sides of the rule (2 n N <= 3 x 148 x 4096) equal single products."""
+    require_gpu()
+    import aoa_b200 as aoa
+    ps = _primes("mixed", 14, 9)
+    E = aoa.Engine(14, ps[:4], ps[4:])
+    E.tune("batch_streams", 1)
+    E.tune("ntt_waves", 1)                       # the two-pass kernels
+    ctx = aoa.Context(E)
+    rng = np.random.default_rng(n)
+    evk = aoa.SwitchKey(ctx, uniform_residues(rng, ps, E.N), uniform_residues(rng, ps, E.N))
+    cts = []
+    for _ in range(3):
+        h = (uniform_residues(rng, ps[:4], E.N), uniform_residues(rng, ps[:4], E.N))
+        cts.append(aoa.Ciphertext.from_residues(ctx, *h, slots=8, scale=SCALE, domain=aoa.AOA_NTT))
+        cts[-1].set(m - 1, 8, SCALE, aoa.AOA_NTT)
+    a, b = [cts[i % 3] for i in range(n)], [cts[i % 2] for i in range(n)]
+    outs = [aoa.Ciphertext(ctx) for _ in range(n)]
+    aoa.ckks_mul_batch(ctx, outs, a, b, evk)
+    one = aoa.Ciphertext(ctx)
+    for i in (0, 1, 5, n - 1):
+        aoa.ckks_mul(ctx, one, a[i], b[i], evk)
+        want, got = one.download(nlimbs=m - 1, domain=aoa.AOA_COEF), outs[i].download(nlimbs=m - 1, domain=aoa.AOA_COEF)
+        assert np.array_equal(want[0], got[0]) and np.array_equal(want[1], got[1])
