@@ -14,6 +14,7 @@
 #include <functional>
 
 #include "aoa_internal.h"
+#include "tune_sample.h"
 
 namespace aoa {
 namespace {
@@ -54,10 +55,9 @@ extern "C" int aoa_engine_autotune(aoa_engine* h, int limbs, char* report, size_
     if (E.log_n < 10) throw AoaError(AOA_ERR_BAD_PARAM, "autotune: ring too small for the two-pass transform");
     const long N = E.N;
     const int k = E.k;
-    // about 12x the L2 size by default, in whole polys of k limbs
-    const long want = limbs > 0 ? limbs : std::max<long>(k, (1536L << 20) / (8 * N));
-    const int npolys = (int)std::max<long>(1, (want + k - 1) / k);
-    const long words = (long)npolys * k * N;
+    const TuneSample sample = tune_sample(limbs, k, N);
+    const int npolys = (int)sample.npolys, half = sample.half;
+    const long words = sample.polys * k * N;
     AOA_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     AOA_CUDA(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking));
     AOA_CUDA(cudaMalloc(&buf, words * 8));
@@ -72,7 +72,6 @@ extern "C" int aoa_engine_autotune(aoa_engine* h, int limbs, char* report, size_
     // the two halves of a batched HMult of 16 run their transforms), so
     // that a shape that only pays off on very large calls does not win.
     // Each figure is the best of two timings.
-    const int half = std::max(1, std::min(npolys / 2, 8));
     auto time_polys = [&](int np, int reps, bool two) -> float {
       float best_ms = 0;
       for (int t = 0; t < 3; t++) {                  // warm-up, then two timed runs
