@@ -47,11 +47,11 @@ class Engine:
     def tune(self, knob, value):
         """Set a launch-shape knob ("ntt_split", "dgt_split", "ntt_cols_div", "ntt_cols_kind",
         "ntt_rows_div", "ntt_waves", "ntt_waves_large", "ntt_chunk_bytes",
-        "ntt_cols_tma", "conv_tensor_cores", "fuse", "batch_streams", "spin_limit")."""
+        "ntt_cols_tma", "ntt_whole", "conv_tensor_cores", "fuse", "batch_streams", "spin_limit")."""
         capi.check(capi.load().aoa_engine_tune(self.handle, knob.encode(), float(value)))
 
     TRANSFORM_KNOBS = ("ntt_split", "ntt_cols_div", "ntt_cols_kind", "ntt_rows_div", "ntt_waves",
-                       "ntt_waves_large", "ntt_chunk_bytes")
+                       "ntt_waves_large", "ntt_chunk_bytes", "ntt_whole")
 
     def tune_get(self, knob):
         """Current value of a launch-shape knob."""

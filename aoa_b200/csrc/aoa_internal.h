@@ -60,7 +60,10 @@ struct Tune {
   double ntt_waves = 1.0;             // transform CTAs per pass, in resident waves
   double ntt_waves_large = 8.0;       // the same for launches of at least kLargeItems limbs
   bool conv_tensor_cores = true;      // basis conversion on the int8 tensor cores where it applies
-  bool ntt_shape_set = false;         // a caller chose a shape: no whole-limb kernels
+  // whole-limb kernels for the calls they are faster on (limb_serves): 0 never,
+  // 1 while the shape knobs are at their defaults (a shape that a caller chose
+  // is for every call), 2 whatever those are
+  int ntt_whole = 1;
   int ntt_split = 0;                  // log2(C) - floor(log2(N) / 2) of the R x C transform split
   // the same for the DGT's cyclic limb transforms (N/2 points): at N = 2^16
   // the 2^15-point transforms ran 2-3% faster with 256-point rows than with
@@ -82,7 +85,15 @@ struct Tune {
   // kErrWaitTimeout in the error word and returns (aoa_ctx_sync then reports
   // AOA_ERR_TIMEOUT); the default 2^20 polls is far beyond any healthy wait
   int spin_limit = 1 << 20;
+
+  bool default_shape() const;         // every shape knob of the two passes at its default
 };
+inline bool Tune::default_shape() const {
+  const Tune d;
+  return ntt_chunk_bytes == d.ntt_chunk_bytes && ntt_waves == d.ntt_waves && ntt_waves_large == d.ntt_waves_large &&
+         ntt_split == d.ntt_split && dgt_split == d.dgt_split && ntt_cols_div == d.ntt_cols_div &&
+         ntt_cols_kind == d.ntt_cols_kind && ntt_rows_div == d.ntt_rows_div && ntt_cols_tma == d.ntt_cols_tma;
+}
 
 // Device copy of the basis-conversion / rescale constants.
 struct RnsTables {

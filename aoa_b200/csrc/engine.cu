@@ -347,6 +347,7 @@ int aoa_engine_tune(aoa_engine* h, const char* knob, double value) {
   else if (k == "dgt_split" && value >= -2 && value <= 2 && value == (int)value) h->e.tune.dgt_split = (int)value;
   else if (k == "ntt_cols_div" && value >= 0 && value <= 2 && value == (int)value) h->e.tune.ntt_cols_div = (int)value;
   else if (k == "ntt_rows_div" && value >= 0 && value <= 2 && value == (int)value) h->e.tune.ntt_rows_div = (int)value;
+  else if (k == "ntt_whole" && value >= 0 && value <= 2 && value == (int)value) h->e.tune.ntt_whole = (int)value;
   else if (k == "ntt_cols_kind" && (value == 0 || value == 1)) h->e.tune.ntt_cols_kind = (int)value;
   else if (k == "batch_streams" && (value == 1 || value == 2)) h->e.tune.batch_streams = (int)value;
   else if (k == "fuse" && value >= 0 && value <= 7 && value == (int)value) h->e.tune.fuse = (int)value;
@@ -354,7 +355,6 @@ int aoa_engine_tune(aoa_engine* h, const char* knob, double value) {
   else if (k == "spin_limit" && value >= 0 && value <= (1 << 30) && value == (int)value)
     h->e.tune.spin_limit = (int)value;
   else return fail(AOA_ERR_BAD_PARAM, "unknown knob or value out of range: " + k);
-  if (k.rfind("ntt_", 0) == 0 || k == "dgt_split") h->e.tune.ntt_shape_set = true;
   return AOA_OK;
 }
 
@@ -375,6 +375,7 @@ int aoa_engine_tune_get(const aoa_engine* h, const char* knob, double* value) {
   else if (k == "fuse") *value = t.fuse;
   else if (k == "spin_limit") *value = t.spin_limit;
   else if (k == "ntt_cols_tma") *value = t.ntt_cols_tma;
+  else if (k == "ntt_whole") *value = t.ntt_whole;
   else return fail(AOA_ERR_BAD_PARAM, "unknown knob: " + k);
   return AOA_OK;
 }

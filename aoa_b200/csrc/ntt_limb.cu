@@ -577,7 +577,8 @@ void limb_init(const Engine&) {
 // a line each.
 bool limb_serves(const Engine& E, int log_n, long items, bool fused) {
   constexpr long kMost[2][6] = {{1024, 1024, 448, 128, 64, 8}, {1024, 1024, 320, 112, 56, 20}};   // log_n = 10 .. 15
-  return !E.tune.ntt_shape_set && log_n >= 10 && log_n <= 15 && items <= kMost[fused][log_n - 10];
+  const bool on = E.tune.ntt_whole == 2 || (E.tune.ntt_whole == 1 && E.tune.default_shape());
+  return on && log_n >= 10 && log_n <= 15 && items <= kMost[fused][log_n - 10];
 }
 
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,

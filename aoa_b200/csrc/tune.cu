@@ -121,6 +121,7 @@ extern "C" int aoa_engine_autotune(aoa_engine* h, int limbs, char* report, size_
          [](const Tune& t) { return (double)t.ntt_chunk_bytes; },
          [](Tune& t, double v) { t.ntt_chunk_bytes = (long)v; }},
     };
+    E.tune.ntt_whole = 0;                            // these shapes are the two-pass kernels'
     float best = time_once();
     char line[256];
     snprintf(line, sizeof line, "{\"limbs\": %ld, \"start_ms\": %.4f, \"trials\": [", (long)npolys * k, best);
@@ -147,11 +148,14 @@ extern "C" int aoa_engine_autotune(aoa_engine* h, int limbs, char* report, size_
     // others have changed
     for (int round = 0; round < 2; round++)
       for (const Knob& kn : knobs) descend(kn);
+    // small calls keep the whole-limb kernels beside whatever shape was chosen
+    E.tune.ntt_whole = saved.ntt_whole == 1 && saved.default_shape() ? 2 : saved.ntt_whole;
     snprintf(line, sizeof line,
              "], \"best_ms\": %.4f, \"choice\": {\"ntt_split\": %d, \"ntt_cols_div\": %d, \"ntt_cols_kind\": %d, "
-             "\"ntt_rows_div\": %d, \"ntt_waves\": %g, \"ntt_waves_large\": %g, \"ntt_chunk_bytes\": %ld}}",
+             "\"ntt_rows_div\": %d, \"ntt_waves\": %g, \"ntt_waves_large\": %g, \"ntt_chunk_bytes\": %ld, "
+             "\"ntt_whole\": %d}}",
              best, E.tune.ntt_split, E.tune.ntt_cols_div, E.tune.ntt_cols_kind, E.tune.ntt_rows_div, E.tune.ntt_waves,
-             E.tune.ntt_waves_large, E.tune.ntt_chunk_bytes);
+             E.tune.ntt_waves_large, E.tune.ntt_chunk_bytes, E.tune.ntt_whole);
     rep += line;
   });
   if (st_ != AOA_OK) E.tune = saved;

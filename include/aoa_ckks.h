@@ -110,9 +110,12 @@ int aoa_engine_destroy(aoa_engine* e);
  * "spin_limit" (polls of the kernels' bounded mbarrier waits before they
  * give up and report AOA_ERR_TIMEOUT at the next aoa_ctx_sync, 0..2^30;
  * default 2^20; the drain of copies and MMAs in flight after an expired
- * wait always uses the default bound).  Rings up to 2^14 run small calls as
- * one whole-limb kernel per transform, which has no shape to choose: setting
- * any "ntt_*" knob or "dgt_split" keeps the engine on the two-pass kernels. */
+ * wait always uses the default bound).  Rings up to 2^15 run small calls as
+ * one whole-limb kernel per transform, which has no shape to choose:
+ * "ntt_whole" 1 (the default) does so while every other "ntt_*" knob and
+ * "dgt_split" is at its default, so that a shape chosen here is every call's;
+ * 0 keeps every call on the two-pass kernels, 2 keeps the whole-limb kernels
+ * beside a chosen shape.                                                    */
 int aoa_engine_tune(aoa_engine* e, const char* knob, double value);
 /* current value of a knob (names as for aoa_engine_tune) */
 int aoa_engine_tune_get(const aoa_engine* e, const char* knob, double* value);
@@ -124,7 +127,10 @@ int aoa_engine_tune_get(const aoa_engine* e, const char* knob, double* value);
  * (coordinate descent from the current setting; a change is kept when it
  * is at least 2% faster), keeps the best and writes
  * a JSON report of the choice and the objective values (ms) into
- * report[0 .. report_len) (report may be NULL).  Run it before
+ * report[0 .. report_len) (report may be NULL).  Every trial runs the
+ * two-pass kernels, whose shapes these are; small calls keep the whole-limb
+ * kernels if they had them before ("ntt_whole" 2 in the choice, so that setting
+ * the reported knobs gives the tuned engine again).  Run it before
  * the engine is used from other streams; it synchronises the device.       */
 int aoa_engine_autotune(aoa_engine* e, int limbs, char* report, size_t report_len);
 /* ring degree, prime count, primes (out may be NULL) */

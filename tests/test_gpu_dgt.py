@@ -69,6 +69,7 @@ def test_dgt_split_knob_keeps_results(dgt_table, log_n):
     require_gpu()
     aoa, E, ctx, D, _ = _setup(dgt_table, log_n, 3, 2, 55)
     assert E.tune_get("dgt_split") == 1
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     rng = np.random.default_rng(log_n + 3)
     x = uniform_residues(rng, E.primes, E.N)
     want = unfold(D.fwd(fold(x)))

@@ -56,6 +56,7 @@ def test_zero_spin_limit_in_transform_kernels_reports_timeout(cols_kind):
     (both column-pass kinds), drain the copy in flight and return."""
     require_gpu()
     aoa, E, ctx, o, Q, B = _setup()
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     E.tune("ntt_cols_kind", cols_kind)
     rng = np.random.default_rng(2)
     x = np.stack([uniform_residues(rng, Q + B, E.N) for _ in range(4)])

@@ -20,7 +20,7 @@ def test_transforms_at_the_lazy_prime_bounds(log_n, top):
     ps = (params.ntt_primes(60, 2 << log_n, 1) + params.ntt_primes(35, 2 << log_n, 1)
           + params.ntt_primes(34, 2 << log_n, 1) + params.ntt_primes(60, 1 << 32, 1))
     E = aoa.Engine(log_n, ps[:3], ps[3:])
-    E.tune("ntt_waves", 1)                       # the two-pass kernels
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     ctx, o = aoa.Context(E), Oracle(E.N, ps[:3], ps[3:])
     x = uniform_residues(np.random.default_rng(log_n), ps, E.N)
     if top:
@@ -47,7 +47,7 @@ def test_inverse_sums_at_the_lazy_prime_bounds(log_n, whole_limb):
           + params.ntt_primes(35, 2 << log_n, 1) + params.ntt_primes(62, 2 << log_n, 1))
     E = aoa.Engine(log_n, ps[:2], ps[2:])
     if not whole_limb:
-        E.tune("ntt_waves", 1)                   # the two-pass kernels
+        E.tune("ntt_whole", 0)                   # the two-pass kernels
     ctx, o = aoa.Context(E), Oracle(E.N, ps[:2], ps[2:])
     top = np.array(ps, dtype=np.uint64)[:, None] - np.uint64(1)
     for span in [0, 1, 2, 8, 64, E.N // 4, E.N // 2]:

@@ -75,7 +75,7 @@ def test_hmult_and_rotations_equal_the_two_pass_kernels(log_n, k, n, rescale):
         return res + [x.download(domain=aoa.AOA_NTT) for x in rot]
 
     whole = run(False) + run(True)
-    E.tune("ntt_waves", 1)                       # a chosen shape: the two-pass kernels
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     passes = run(False)
     for i, w in enumerate(whole):
         p = passes[i % len(passes)]
@@ -99,3 +99,51 @@ def test_expired_waits_are_reported_and_the_context_recovers():
     d = ctx.upload(x)
     ctx.ntt_fwd(d, 1, 0, 6)
     assert np.array_equal(d.numpy(), o.ntt_fwd(x))
+
+
+def test_launch_shapes_choose_between_the_kernels():
+    """A shape knob moves every call to the two passes while it differs from its default and no longer;
+    "ntt_whole" overrides either way; the tuner times the two passes, leaves the small calls as they were, and
+    its reported choice set on another engine gives the same launches."""
+    require_gpu()
+    import aoa_b200 as aoa
+    Q, B = _primes(12, 4, 5)
+    E = aoa.Engine(12, Q, B)
+
+    def launches(E):
+        ctx = aoa.Context(E)
+        d = ctx.upload(np.zeros((4, E.N), dtype=np.uint64))
+        n0 = aoa.kernel_launches()
+        ctx.ntt_fwd(d, 1, 0, 4)
+        ctx.ntt_inv(d, 1, 0, 4)
+        n = aoa.kernel_launches() - n0
+        ctx.sync()
+        return n
+
+    assert launches(E) == 2
+    shapes = {"ntt_split": 1, "dgt_split": 0, "ntt_cols_div": 1, "ntt_rows_div": 0, "ntt_cols_kind": 1,
+              "ntt_cols_tma": 0, "ntt_waves": 2, "ntt_waves_large": 2, "ntt_chunk_bytes": 1 << 30}
+    two = {}
+    for knob, value in shapes.items():
+        default = E.tune_get(knob)
+        E.tune(knob, default)
+        assert launches(E) == 2, knob            # the default value chooses nothing
+        E.tune(knob, value)
+        two[knob] = launches(E)
+        E.tune("ntt_whole", 2)
+        assert launches(E) == 2, knob
+        E.tune("ntt_whole", 1)
+        E.tune(knob, default)
+        assert two[knob] >= 4 and launches(E) == 2, knob
+    E.tune("ntt_whole", 0)
+    assert launches(E) >= 4
+    E.tune("ntt_whole", 1)
+    n0 = aoa.kernel_launches()
+    rep = E.autotune(limbs=64)
+    # every figure: three runs of two forward + inverse pairs and of four on each of two streams
+    assert aoa.kernel_launches() - n0 >= (len(rep["trials"]) + 1) * 3 * (2 * 2 + 4 * 4) * 2
+    assert launches(E) == 2
+    E2 = aoa.Engine(12, Q, B)
+    for knob, value in rep["choice"].items():
+        E2.tune(knob, value)
+    assert launches(E2) == 2 and E2.transform_shapes() == E.transform_shapes()

@@ -100,6 +100,7 @@ def test_ntt_launch_shapes_bit_exact(log_n, shape):
     split, cdiv, rdiv, kind = shape
     ps = oracle.gen_ntt_primes(60, 2 << log_n, 3)
     E, ctx, o = _engine_and_oracle(log_n, ps[:2], ps[2:])
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     E.tune("ntt_split", split)
     E.tune("ntt_cols_div", cdiv)
     E.tune("ntt_rows_div", rdiv)
@@ -126,6 +127,7 @@ def test_ntt_prime_size_edges(bits, shape):
     log_n = 15
     ps = oracle.gen_ntt_primes(bits, 1 << 17, 4)
     E, ctx, o = _engine_and_oracle(log_n, ps[:2], ps[2:])
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     E.tune("ntt_split", split)
     E.tune("ntt_cols_kind", kind)
     rng = np.random.default_rng(bits + 10 * (split + 2) + 100 * kind)
@@ -151,6 +153,7 @@ def test_column_tiles_by_tensor_map_equal_row_copies(log_n, split, src):
     import aoa_b200 as aoa
     ps = oracle.gen_ntt_primes(60, 2 << log_n, 5)
     E, ctx, o = _engine_and_oracle(log_n, ps[:3], ps[3:])
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     E.tune("ntt_split", split)
     E.tune("ntt_chunk_bytes", max(1 << 20, 2 * 4 * (8 << log_n)))   # two polys per launch pair from 2^15
     rng = np.random.default_rng(log_n + 3 * split)
@@ -189,6 +192,7 @@ def test_autotune_keeps_results_bit_exact():
     ch = rep["choice"]
     assert -2 <= ch["ntt_split"] <= 2 and 0 <= ch["ntt_cols_div"] <= 2 and 0 <= ch["ntt_rows_div"] <= 2
     assert rep["best_ms"] <= rep["start_ms"] * 1.0001 and len(rep["trials"]) >= 10
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     rng = np.random.default_rng(11)
     x = _rand(rng, ps, 1 << 14, npolys=2)
     d = ctx.upload(x)
@@ -238,6 +242,7 @@ def test_primes_one_mod_2_32_take_the_short_remainder(log_n, shape):
     assert all(q % (1 << 32) == 1 and q < 1 << 60 for q in q1) and len(lazy) == 2
     ps = [q1[0], lazy[0], q1[1], big[0], q1[2], lazy[1], big[1]]
     E, ctx, o = _engine_and_oracle(log_n, ps[:5], ps[5:])
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     E.tune("ntt_split", split)
     E.tune("ntt_cols_div", cdiv)
     E.tune("ntt_rows_div", rdiv)
@@ -258,6 +263,7 @@ def test_primes_one_mod_2_32_take_the_short_remainder(log_n, shape):
     assert np.array_equal(dy.numpy()[0], o.ntt_inv(y[0]))
     # a set of such primes only (one run per pass, as in the benchmark)
     E1, ctx1, o1 = _engine_and_oracle(log_n, q1[:2], q1[2:])
+    E1.tune("ntt_whole", 0)
     x1 = _rand(rng, q1, n, npolys=2)
     d1 = ctx1.upload(x1)
     ctx1.ntt_fwd(d1, 2, 0, 3)

@@ -65,7 +65,7 @@ def test_rescaled_limb_joins_the_special_limbs_up_to_one_wave(n, m):
     ps = _primes("mixed", 14, 9)
     E = aoa.Engine(14, ps[:4], ps[4:])
     E.tune("batch_streams", 1)
-    E.tune("ntt_waves", 1)                       # the two-pass kernels
+    E.tune("ntt_whole", 0)                       # the two-pass kernels
     ctx = aoa.Context(E)
     rng = np.random.default_rng(n)
     evk = aoa.SwitchKey(ctx, uniform_residues(rng, ps, E.N), uniform_residues(rng, ps, E.N))
