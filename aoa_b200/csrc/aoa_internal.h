@@ -40,11 +40,7 @@ constexpr unsigned kErrWaitTimeout = 1u;   // an mbarrier wait hit its iteration
 #define AOA_LAZY_PRIME_BITS 60
 #endif
 constexpr int kLazyPrimeBits = AOA_LAZY_PRIME_BITS;
-// and above 2^34: their conditional subtractions compare high words only, which
-// leaves up to 2^32 of excess for the last, exact one (smaller primes, which no
-// 64-bit limb is used for in earnest, take canonical butterflies too)
-constexpr uint64_t kLazyPrimeMin = 1ull << 34;
-__host__ __device__ inline bool lazy_prime(uint64_t q) { return q >= kLazyPrimeMin && q < (1ull << kLazyPrimeBits); }
+__host__ __device__ inline bool lazy_prime(uint64_t q) { return q < (1ull << kLazyPrimeBits); }
 constexpr int kButterflyCanonical = 0, kButterflyLazy = 1, kButterflyLazyQ1 = 2;
 // Output primes from here up take one 32-bit Montgomery step in the tensor-core
 // conversion's epilogue (its result is below q + 2^49)

@@ -162,11 +162,14 @@ struct Bf {
     x = U + V;
     y = mulw(U - V + (q << 3), w, q);
   }
-  static __device__ __forceinline__ uint64_t fwd_out(uint64_t x, uint64_t q) {   // [0, 16q + 2^32) -> [0, q)
-    x = csub_hi(x, q << 3);
+  // forward result to [0, q): exactly for the general kind, whose primes may be
+  // of any size (high words there: 198.8 us against 196.7 for 240 limbs at 2^16)
+  static __device__ __forceinline__ uint64_t fwd_out(uint64_t x, uint64_t q) {
+    if constexpr (KIND == kButterflyLazy) return csub(csub(csub(csub(x, q << 3), q << 2), q << 1), q);   // [0, 16q)
+    x = csub_hi(x, q << 3);                     // [0, 16q + 2^32)
     x = csub_hi(x, q << 2);
     x = csub_hi(x, q << 1);                     // [0, 2q + 2^32)
-    x = csub(x, q);                             // [0, q + 2^32), 2^32 < q
+    x = csub(x, q);                             // [0, q + 2^32), 2^32 < q = 1 mod 2^32
     return csub(x, q);
   }
 };
