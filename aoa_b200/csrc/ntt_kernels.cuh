@@ -30,6 +30,7 @@
 
 #include "aoa_internal.h"
 #include "async.cuh"
+#include "ntt_grid.h"
 
 namespace aoa {
 
@@ -892,17 +893,12 @@ ntt_rows(NttBatch b, const __grid_constant__ NttEpi epi) {
 
 // ---- host launchers ----------------------------------------------------------
 
-// CTAs per tile column: about one resident wave of CTAs (blocks_per_sm per SM)
+// large launches balance better with more, shorter-lived CTAs (the hardware
+// hands later waves to the SMs that finish first); small ones pay per CTA
 static inline int ctas_per_tile(const Engine& E, int tiles, int items, int blocks_per_sm) {
-  // Calls of up to two and a half waves run one tile per CTA: with one wave of
-  // CTAs some of them hold two tiles and some three (31 limbs in 27 groups at
-  // 2^16: two for 4 groups, one for 23), and the pass ends with the longest.
-  if ((double)items * tiles <= 2.5 * E.num_sms * blocks_per_sm) return items;
-  // large launches balance better with more, shorter-lived CTAs (the hardware
-  // hands later waves to the SMs that finish first); small ones pay per CTA
-  const double waves = items >= kLargeItems ? E.tune.ntt_waves_large : E.tune.ntt_waves;
-  const int target = std::max(1, (int)(waves * E.num_sms * blocks_per_sm) / std::max(1, tiles));
-  return std::max(1, std::min(items, target));
+  const bool large = items >= kLargeItems;
+  return ctas_per_tile(large ? E.tune.ntt_waves_large : E.tune.ntt_waves,
+                       large ? Tune{}.ntt_waves_large : Tune{}.ntt_waves, E.num_sms * blocks_per_sm, tiles, items);
 }
 
 // The column pass's tile as a 4-D tensor map over the launch's limbs: (column,

@@ -302,3 +302,42 @@ def test_mixed_prime_sizes_run_lazy_and_strict_limbs(log_n):
     for p in range(3):
         assert np.array_equal(X[p, 2:6], o.ntt_fwd(x[p, 2:6], first=2)), p
         assert np.array_equal(X[p, :2], x[p, :2]) and np.array_equal(X[p, 6:], x[p, 6:])
+
+
+@pytest.mark.parametrize("log_n,split", [(11, 0), (14, -1), (16, 0)])
+@pytest.mark.parametrize("cols_kind,tma", [(0, 1), (0, 0), (1, 1)])
+def test_ctas_that_loop_over_limbs_of_several_primes(log_n, split, cols_kind, tma):
+    """One CTA per tile column (a hundredth of a wave): each transforms every poly of every prime of a butterfly
+    kind in turn, so that both tile buffers refill, the barriers' phases wrap and the twiddles change hands; also
+    HMult's inverses without N^-1, whose first limb is not under the prime before the second's."""
+    require_gpu()
+    import aoa_b200 as aoa
+    from tests.ckks_inputs import make_keys
+    n = 1 << log_n
+    q1 = oracle.gen_ntt_primes(60, 1 << 32, 4)
+    lazy = oracle.gen_ntt_primes(55, 2 * n, 4)
+    big = oracle.gen_ntt_primes(62, 2 * n, 3)
+    for ps in (q1[:3] + lazy[:3] + big, q1 + lazy):
+        k = 4
+        E, ctx, o = _engine_and_oracle(log_n, ps[:k], ps[k:])
+        for knob, value in (("ntt_waves", 0.01), ("ntt_split", split), ("ntt_cols_kind", cols_kind),
+                            ("ntt_cols_tma", tma)):
+            E.tune(knob, value)
+        rng = np.random.default_rng(log_n + cols_kind)
+        x = _rand(rng, ps, n, npolys=2)
+        x[1] = np.array([[p - 1] * n for p in ps], dtype=np.uint64)
+        d = ctx.upload(x)
+        ctx.ntt_fwd(d, 2, 0, len(ps))
+        X = d.numpy()
+        assert all(np.array_equal(X[p], o.ntt_fwd(x[p])) for p in range(2))
+        ctx.ntt_inv(d, 2, 0, len(ps))
+        assert np.array_equal(d.numpy(), x)
+        keys = make_keys(o, seed=3)
+        a, b = [aoa.Ciphertext.from_residues(ctx, y[0, :k], y[1, :k], slots=4, scale=1 << 40, domain=aoa.AOA_NTT)
+                for y in (x, X)]
+        out = aoa.Ciphertext(ctx)
+        aoa.ckks_mul(ctx, out, a, b, aoa.SwitchKey(ctx, *keys["evk"]))
+        w0, w1, _ = o.hmult((x[0, :k], x[1, :k]), (X[0, :k], X[1, :k]), keys["evk"], k - 1, 1 << 40, 1 << 40,
+                            rescale=True, a_state=oracle.ST_NTT, b_state=oracle.ST_NTT)
+        g0, g1 = out.download(nlimbs=k - 1, domain=aoa.AOA_COEF)
+        assert np.array_equal(g0, w0[:k - 1]) and np.array_equal(g1, w1[:k - 1])
