@@ -94,7 +94,7 @@ int aoa_engine_destroy(aoa_engine* e);
  * compile-time constants): "ntt_chunk_bytes" (bytes of limbs per transform
  * launch pair, default 4 GiB),
  * "ntt_waves" (transform CTAs per pass in resident waves, default 1: at that
- * value calls of up to two and a half waves of tiles run a CTA per tile),
+ * value small calls run a CTA per tile),
  * "ntt_waves_large" (the same for launches of at least 1536 limbs, default 8),
  * "ntt_split" (log2 C - floor(log2 N / 2) of the R x C transform split,
  * -2..2, default 0), "dgt_split" (the same for the DGT's N/2-point cyclic

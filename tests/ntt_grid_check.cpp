@@ -11,11 +11,12 @@ int main() {
       for (int items = 1; items <= 3000; items += 1 + items / 8)
         for (double waves : {0.01, 0.5, 1.0, 2.0, 2.5, 8.0, 64.0})
           for (double def : {1.0, 8.0}) {
-            const int g = aoa::ctas_per_tile(waves, def, resident, tiles, items);
+            const double apart = items % 2 ? aoa::cols_apart() : aoa::rows_apart(1 + items % 3);
+            const int g = aoa::ctas_per_tile(waves, def, apart, resident, tiles, items);
             const double want = waves * resident / tiles;   // CTAs per tile column of that many waves
             bool ok = g >= 1 && g <= items;
-            if (waves != def) ok = ok && (g == items ? want >= items : g <= want || g == 1) && (g == items || g + 1 > want);
-            else if (items * (double)tiles <= 2.5 * resident) ok = ok && g == items;
+            if (waves == def && items * (double)tiles <= apart * resident) ok = ok && g == items;
+            else ok = ok && (g == 1 || g <= want) && (g == items || g + 1 > want);
             if (!ok) {
               std::printf("waves %g (default %g), resident %d, tiles %d, items %d: %d\n", waves, def, resident, tiles,
                           items, g);
