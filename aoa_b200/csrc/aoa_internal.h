@@ -309,11 +309,14 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
 void ntt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int nlimbs,
                long poly_stride, bool forward, cudaStream_t st);
 
-// ntt_limb.cu: whole-limb transforms of N = 2^10 .. 2^14 and the ends of HMult and
+// ntt_limb.cu: whole-limb transforms of N = 2^10 .. 2^15 and the ends of HMult and
 // the automorphisms fused with them.  limb_serves: whether a call of `items`
-// limb transforms (plain, or the fused ends of a key switch) takes them.
+// limb transforms takes them: a forward transform of limbs of one lazy kind, the
+// DGT's cyclic transforms of one lazy kind, any other transform, or the fused ends
+// of a key switch.
+enum LimbUse { kLimbForward, kLimbCyclic, kLimbOther, kLimbFused };
 void limb_init(const Engine& E);
-bool limb_serves(const Engine& E, int log_n, long items, bool fused);
+bool limb_serves(const Engine& E, int log_n, long items, LimbUse use);
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,
                     long poly_stride, bool forward, const NttIo& io, cudaStream_t st);
 // D2 + z half = a1 b1 and T + z half = its unscaled inverse transform, op z

@@ -291,8 +291,9 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
     for (int z = 0; z < n; z++) late = late && (x == z || (out[x] != a[z] && out[x] != b[z]));
   // small rings: five launches, the transforms as whole-limb clusters with the
   // work around them inside (ntt_limb.cu)
-  const bool whole = late && tk == AOA_NTT && fuse == kFuseSource && limb_serves(E, E.log_n, 2L * n * (kl + 1), true) &&
-                     limb_serves(E, E.log_n, 2L * n * m, true);
+  const bool whole = late && tk == AOA_NTT && fuse == kFuseSource &&
+                     limb_serves(E, E.log_n, 2L * n * (kl + 1), kLimbFused) &&
+                     limb_serves(E, E.log_n, 2L * n * m, kLimbFused);
   if (whole) {
     limb_tensor_inv(E, ptr, half, D2, T, n, m, st);
     modup(E, T, half, UB, (long)kl * N, n, level, st, true);
@@ -586,8 +587,8 @@ static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* co
       out[z]->domain = AOA_NTT;
     }
   };
-  if (E.tune.fuse == kFuseSource && limb_serves(E, E.log_n, 2L * n * kl, true) &&
-      limb_serves(E, E.log_n, 2L * n * m, true)) {
+  if (E.tune.fuse == kFuseSource && limb_serves(E, E.log_n, 2L * n * kl, kLimbFused) &&
+      limb_serves(E, E.log_n, 2L * n * m, kLimbFused)) {
     // small rings: whole-limb clusters (as hmult_group)
     limb_galois_inv(E, ptr, gl, half, R, T, n, m, st);
     modup(E, T, half, UB, (long)kl * N, n, level, st, true);

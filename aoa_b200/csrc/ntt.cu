@@ -87,6 +87,15 @@ static void check_alignment(const uint64_t* data, const NttIo* io) {
     throw AoaError(AOA_ERR_BAD_PARAM, "ntt: device data must be 16-byte aligned");
 }
 
+static LimbUse limb_use(const NttTables& T, int first_prime, int nlimbs, int gap, bool forward) {
+  auto kind_at = [&](int l) {
+    return T.prime_kind ? (int)T.prime_kind[first_prime + (l >> T.prime_shift) + (l ? gap : 0)] : T.kind;
+  };
+  bool one_lazy = kind_at(0) != kButterflyCanonical;
+  for (int l = 1; l < nlimbs && one_lazy && T.prime_kind; l++) one_lazy = kind_at(l) == kind_at(0);
+  return !one_lazy ? kLimbOther : T.prime_shift ? kLimbCyclic : forward ? kLimbForward : kLimbOther;
+}
+
 // Transform limbs [0, nlimbs) of npolys polys (layout [npolys][poly_stride][N],
 // N = 2^T.log_n) with the tables T; limb l under prime first_prime +
 // (l >> T.prime_shift).  Large transforms are split into chunks of whole polys
@@ -97,7 +106,8 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
   const int gap = io && nlimbs > 1 ? io->prime_gap : 0;
   if (first_prime < 0 || first_prime + ((nlimbs - 1) >> T.prime_shift) + gap >= E.nprimes)
     throw AoaError(AOA_ERR_BAD_PARAM, "ntt: prime range out of bounds");
-  if (limb_serves(E, T.log_n, (long)npolys * nlimbs, false) && (!io || io->epi.mode == kEpiStore)) {
+  if ((!io || io->epi.mode == kEpiStore) &&
+      limb_serves(E, T.log_n, (long)npolys * nlimbs, limb_use(T, first_prime, nlimbs, gap, forward))) {
     check_alignment(data, io);
     limb_transform(E, T, data, npolys, first_prime, nlimbs, poly_stride, forward, io ? *io : NttIo{}, st);
     return;

@@ -564,21 +564,33 @@ void limb_init(const Engine&) {
 }
 
 // Up to how many limb transforms the whole-limb kernels are faster than the two
-// passes, which have the higher throughput once the chip is full.  Measured
-// (us, two passes -> whole limbs, one B200): forward + inverse of 8 limbs
-// 12.1 -> 6.9 at 2^10, 13.7 -> 9.0 at 2^12, 21.4 -> 19.5 at 2^14; of 64 limbs
-// 20.6 -> 11.9 at 2^12, 50.0 -> 42.4 at 2^14; of 256 limbs 31.1 -> 19.8 at 2^11,
-// 44.0 -> 35.9 at 2^12, 69.0 -> 78.3 at 2^13; of 512 limbs 65.2 -> 66.1 at 2^12;
-// HMult with 12 limbs (28 key-product limbs) 55.3 -> 34.9 at 2^12, 97.8 -> 63.6
-// at 2^14, 124.5 -> 121.7 at 2^15; four of them (112) 118.8 -> 113.4 at 2^13,
-// 171.6 -> 207.9 at 2^14; rotation with 20 limbs (42) 103.1 -> 99.6 at 2^14,
-// 148.6 -> 189.5 at 2^15.  A plain transform (two launches saved to one) and the
-// fused ends of a key switch (`fused`: its 2 n (kl + 1) key-product limbs) have
-// a line each.
-bool limb_serves(const Engine& E, int log_n, long items, bool fused) {
-  constexpr long kMost[2][6] = {{1024, 1024, 448, 128, 64, 8}, {1024, 1024, 320, 112, 56, 20}};   // log_n = 10 .. 15
+// passes, which have the higher throughput once the chip is full.  Measured on
+// both sides of each line (us, two passes -> whole limbs, one B200):
+//   forward, one lazy kind: 2^11, 1024 limbs 40 -> 31; 2^12, 112 11.1 -> 10.1, 150
+//     12.2 -> 13.3, 336 20.7 -> 23.8; 2^13, 64 13.9 -> 12.3, 80 16.2 -> 16.5, 128
+//     18.4 -> 21.6; 2^14, 32 (a cluster of four on every SM) 12.5 -> 11.0, 36 12.6
+//     -> 21.0, 64 21.4 -> 22.1; 2^15, 1 to 8 8.5 -> 11.0;
+//   DGT limbs of one lazy kind, with the twist: 2^11, 512 22.3 -> 21.6, 608 24.0 ->
+//     26.3; 2^12, 448 forward 37.2 -> 38.7, inverse 41.3 -> 36.2; 2^13, 128 28.3 ->
+//     26.3, 160 31.7 -> 34.1; 2^14, 32 16.1 -> 14.4, 48 18.0 -> 26.2; 2^15, 8 17.4
+//     -> 13.9, 16 19.7 -> 26.5;
+//   other inverses, canonical limbs and calls of several kinds, which take two
+//     launches per kind: inverse of one kind 2^12, 448 30.0 -> 27.8, 672 39.3 ->
+//     40.0; 2^13, 128 21.3 -> 20.1, 160 22.3 -> 24.6; 2^14, 64 24.3 -> 20.5, 80 26.9
+//     -> 30.2; 2^15, 6 8.8 -> 10.6, 8 15.8 -> 10.8, 16 17.4 -> 20.9; forward of
+//     63-bit and 55-bit primes 2^12, 448 35.3 -> 32.0, 672 43.9 -> 46.2; 2^13, 128
+//     35.1 -> 22.8; 2^14, 64 37.0 -> 24.4; 2^15, 8 29.0 -> 13.5;
+//   fused, by the 2 n (kl + 1) key-product limbs of a key switch: HMult 2^12, 320
+//     138 -> 103; 2^13, 110 105 -> 98, 150 120 -> 120, 196 168 -> 179; 2^14, 60 113
+//     -> 94, 100 142 -> 152; rotation 2^14, 56 110 -> 109, 80 136 -> 140; 2^15, 16
+//     83.9 -> 85.8, 24 98 -> 110; HMult 2^15, 20 95 -> 90, 30 107 -> 98.
+bool limb_serves(const Engine& E, int log_n, long items, LimbUse use) {
+  constexpr long kMost[4][6] = {{1024, 1024, 128, 64, 32, 0},     // kLimbForward; log_n = 10 .. 15
+                                {1024, 512, 448, 128, 32, 8},     // kLimbCyclic
+                                {1024, 1024, 448, 128, 64, 8},    // kLimbOther
+                                {1024, 1024, 320, 112, 56, 20}};  // kLimbFused
   const bool on = E.tune.ntt_whole == 2 || (E.tune.ntt_whole == 1 && E.tune.default_shape());
-  return on && log_n >= 10 && log_n <= 15 && items <= kMost[fused][log_n - 10];
+  return on && log_n >= 10 && log_n <= 15 && items <= kMost[use][log_n - 10];
 }
 
 void limb_transform(const Engine& E, const NttTables& T, uint64_t* data, int npolys, int first_prime, int nlimbs,

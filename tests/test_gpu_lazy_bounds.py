@@ -59,8 +59,7 @@ def test_inverse_sums_at_the_lazy_prime_bounds(log_n, whole_limb):
         assert np.array_equal(d.numpy(), o.ntt_inv(x)), span
 
 
-@pytest.mark.parametrize("whole_limb", [False, True])
-@pytest.mark.parametrize("log_n", [11, 14, 15])
+@pytest.mark.parametrize("log_n,whole_limb", [(11, False), (11, True), (14, False), (14, True), (15, False)])
 def test_primes_below_34_bits_are_lazy(log_n, whole_limb):
     """They share the launches of 55-bit primes (a pass runs the limbs of one butterfly kind), and their
     transforms are the oracle's; below 2^31, where the reference's Barrett step is no longer exact, they are
@@ -75,24 +74,21 @@ def test_primes_below_34_bits_are_lazy(log_n, whole_limb):
     ctx, o = aoa.Context(E), Oracle(E.N, ps, [])
     x = np.stack([uniform_residues(np.random.default_rng(log_n), ps, E.N)] * 2)
     x[1] = np.array(ps, dtype=np.uint64)[:, None] - np.uint64(1)
-    limbs = 3 if log_n == 15 else 6              # whole limbs at 2^15: up to 8
-    for first in range(0, 6, limbs):
-        v = x[:, first:first + limbs].copy()
-        d = ctx.upload(v)
-        n0 = aoa.kernel_launches()
-        ctx.ntt_fwd(d, 2, first, limbs)
-        assert aoa.kernel_launches() - n0 == (1 if whole_limb else 2)
-        got = d.numpy()
-        for l, q in enumerate(ps[first:first + limbs]):
-            if q > 1 << 31:
-                want = [o.ntt_fwd(v[p, l:l + 1], first=first + l)[0] for p in range(2)]
-                assert np.array_equal(got[:, l], want), q
-                continue
-            psi = pow(params.primitive_root(q), (q - 1) // n, q)
-            for pos in (0, 1, E.N // 2, E.N - 1):
-                at, value = pow(psi, 2 * bitrev(pos, log_n) + 1, q), 0
-                for c in v[0, l][::-1].tolist():
-                    value = (value * at + c) % q
-                assert got[0, l, pos] == value, (q, pos)
-        ctx.ntt_inv(d, 2, first, limbs)
-        assert np.array_equal(d.numpy(), v)
+    d = ctx.upload(x)
+    n0 = aoa.kernel_launches()
+    ctx.ntt_fwd(d, 2, 0, len(ps))
+    assert aoa.kernel_launches() - n0 == (1 if whole_limb else 2)
+    got = d.numpy()
+    for l, q in enumerate(ps):
+        if q > 1 << 31:
+            want = [o.ntt_fwd(x[p, l:l + 1], first=l)[0] for p in range(2)]
+            assert np.array_equal(got[:, l], want), q
+            continue
+        psi = pow(params.primitive_root(q), (q - 1) // n, q)
+        for pos in (0, 1, E.N // 2, E.N - 1):
+            at, value = pow(psi, 2 * bitrev(pos, log_n) + 1, q), 0
+            for c in x[0, l][::-1].tolist():
+                value = (value * at + c) % q
+            assert got[0, l, pos] == value, (q, pos)
+    ctx.ntt_inv(d, 2, 0, len(ps))
+    assert np.array_equal(d.numpy(), x)
