@@ -21,11 +21,12 @@ inline int ctas_per_tile(double waves, double default_waves, double apart, int r
 // of 2^16 (1.30 waves) 39.1 -> 35.8 forward, 41.1 -> 36.5 inverse, 68 (2.45) 60.7
 // -> 59.9 and 62.7 -> 61.0; 34 of 2^17 105.9 -> 95.5; 240 of 2^14 (2.16) 57.1 ->
 // 52.4).  A row pass that holds the next poly under the same prime keeps its
-// twiddles, which is worth more than the even end from 1.2 waves on: polys of
-// different primes, 16 limbs of 2^16 (1.15) 23.1 -> 21.1, 31 (2.23) 38.7 -> 37.1;
-// three polys each, 33 limbs of 2^16 (2.38) 36.8 -> 40.3; two each, 32 of 2^15
-// (1.15) 26.8 -> 22.3, 50 (1.80) 26.2 -> 28.4, 64 (2.31) 37.6 -> 40.0.
+// twiddles, which soon is worth more than the even end.  One poly: 17 limbs of 2^16
+// (1.23) 24.6 -> 21.4, 31 (2.23) 36.6 -> 35.1.  Two: 20 limbs of 2^16 (1.44) 24.2 ->
+// 23.6, 22 (1.59) 24.3 -> 25.2; 38 of 2^15 (1.37) 25.5 -> 23.6, 50 (1.80) 26.2 ->
+// 28.3.  Eight: 32 of 2^15 (1.15) 23.4 -> 22.0, 40 (1.44) 24.0 -> 26.5, 64 (2.31)
+// 33.0 -> 37.9.
 inline double cols_apart() { return 2.5; }
-inline double rows_apart(int npolys) { return npolys == 1 ? 2.5 : 1.2; }
+inline double rows_apart(int npolys) { return npolys == 1 ? 2.5 : npolys <= 3 ? 1.5 : 1.2; }
 
 }  // namespace aoa
