@@ -273,8 +273,7 @@ struct NttTables {
 //                   (the data is not written)
 //   kEpiCombine     the key-switch epilogue with y = v (ks_combine):
 //                   rescale: ((base + ks B^-1 - v) q_l^-1), else base + (ks - v) B^-1,
-//                   base = 0 for p >= base_polys; written to outp.p[p] (use_ptrs)
-//                   or out + p*out_stride, at l*N + c
+//                   written to outp.p[p] at l*N + c
 enum { kEpiStore = 0, kEpiKeyProduct = 1, kEpiCombine = 2 };
 enum { kFuseSource = 1, kFuseKeyProduct = 2, kFuseCombine = 4 };
 struct NttEpi {
@@ -285,12 +284,10 @@ struct NttEpi {
   long key_half = 0;
   const uint64_t* base = nullptr;
   long base_stride = 0;
-  int base_polys = 0;
   const uint64_t* ks = nullptr;
   long ks_stride = 0;
   const ShoupW* binv = nullptr;
   const ShoupW* resc = nullptr;
-  int use_ptrs = 0;
   OutPtrs outp;
   int limb_base = 0;       // limb of the launch's first limb in out / ks / base
 };
@@ -360,8 +357,6 @@ void dgt_batch(const Engine& E, uint64_t* data, int npolys, int first_prime, int
                bool forward, cudaStream_t st);
 void gi_mul_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* b, long bs,
                int prime0, int nlimbs, int npolys, cudaStream_t st);
-void gi_tensor_op(const Engine& E, const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0,
-                  uint64_t* d1, uint64_t* d2, int nlimbs, cudaStream_t st);
 void gi_keyswitch_mul_op(const Engine& E, const uint64_t* xq, const uint64_t* xb, const uint64_t* key, uint64_t* k0,
                          uint64_t* k1, int nq, cudaStream_t st);
 // the same over a batch of n ops (one launch each)
@@ -377,18 +372,14 @@ void xform(const Engine& E, int kind, uint64_t* d, int npolys, int first_prime, 
 // ops.cu  (op: 0 add, 1 sub, 2 mul, 3 neg)
 void ew_binary_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* b, long bs,
                   int op, int prime0, int nlimbs, int npolys, cudaStream_t st);
-void ew_scalar_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* d_scalars,
-                  int op, int prime0, int nlimbs, int npolys, cudaStream_t st);
 void ew_muladd_op(const Engine& E, uint64_t* d, long ds, const uint64_t* a, long as, const uint64_t* b, long bs,
                   const uint64_t* c, long cs, int prime0, int nlimbs, int npolys, cudaStream_t st);
-void tensor_op(const Engine& E, const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0,
-               uint64_t* d1, uint64_t* d2, int nlimbs, cudaStream_t st);
 void tensor_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D, int n, int nlimbs, cudaStream_t st);
 void keyswitch_mul_batch_op(const Engine& E, const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
                             const uint64_t* key, uint64_t* k, long k_stride, int n, int nq, cudaStream_t st, int nb = -1);
 void ks_combine_ptr(const Engine& E, const OutPtrs& outp, const uint64_t* base, long base_stride, const uint64_t* k,
                     long k_stride, const uint64_t* y, long y_stride, int nlimbs, int npolys, int rescale_level,
-                    cudaStream_t st, int base_polys = -1);
+                    cudaStream_t st);
 // ks_finish.cu: the Q limbs of a key switch in one pass over the operands
 void tensor_d2_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* D2, int n, int nlimbs, cudaStream_t st);
 void hmult_top_op(const Engine& E, const CtPtrs& ptr, long half, const uint64_t* D2, const uint64_t* key, uint64_t* U,
@@ -407,14 +398,10 @@ void galois_finish_op(const Engine& E, const uint64_t* R, long half, const KeyPt
 void automorph_ntt_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint64_t* out, int n,
                             const GaloisList& galois, int nlimbs, cudaStream_t st);
 // key products with a key per op (keys.k[z], [b | a] over all primes)
-void keyswitch_mul_keys_op(const Engine& E, const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
-                           const KeyPtrs& keys, uint64_t* k, long k_stride, int n, int nq, cudaStream_t st);
-void keyswitch_mul_op(const Engine& E, const uint64_t* xq, const uint64_t* xb, const uint64_t* key, uint64_t* k0,
-                      uint64_t* k1, int nq, cudaStream_t st, int nb = -1);
+void keyswitch_mul_keys_op(const Engine& E, const uint64_t* xb, long xb_stride, const KeyPtrs& keys, uint64_t* k,
+                           long k_stride, int n, cudaStream_t st);
 void automorph_coef_op(const Engine& E, uint64_t* out, const uint64_t* in, long poly_stride, long galois,
                        int nlimbs, int npolys, cudaStream_t st);
-void automorph_ntt_op(const Engine& E, uint64_t* out, const uint64_t* in, long poly_stride, long galois,
-                      int nlimbs, int npolys, cudaStream_t st);
 
 // host number theory (primes.cpp)
 uint64_t h_mulmod(uint64_t a, uint64_t b, uint64_t q);

@@ -21,16 +21,16 @@ namespace aoa {
 //   T   [k]          coefficient-domain copy of the key-switch input
 //   UB  [kl]         ModUp output (B limbs)
 //   KS  [2][k + kl]  key products: Q limbs transform domain, B limbs coefficients
-//   L4  [4]          single limbs (d0_l, d1_l, k0_l, k1_l) for the merged rescale
-//   CL  [2]          c_l, limb l of the product in coefficients
 //   Y   [2][k]       ModDown corrections
 //   R0  [k]          automorphism of c0
 struct Workspace {
-  uint64_t *D, *T, *UB, *KS, *L4, *CL, *Y, *R0;
+  uint64_t *D, *T, *UB, *KS, *Y, *R0;
 };
 
+// and six limbs more than that, as much as the batched pipelines need with one
+// operation (batch_words(1), galois_words(1)) at any k
 size_t workspace_words(const Engine& E) {
-  return (size_t)E.N * (3 * E.k + E.k + std::max(E.kl, 1) + 2 * (E.k + E.kl) + 4 + 2 + 2 * E.k + E.k);
+  return (size_t)E.N * (3 * E.k + E.k + std::max(E.kl, 1) + 2 * (E.k + E.kl) + 2 * E.k + E.k + 6);
 }
 
 Workspace carve(const Engine& E, uint64_t* p) {
@@ -40,8 +40,6 @@ Workspace carve(const Engine& E, uint64_t* p) {
   w.T = p; p += E.k * limb;
   w.UB = p; p += std::max(E.kl, 1) * limb;
   w.KS = p; p += 2 * (E.k + E.kl) * limb;
-  w.L4 = p; p += 4 * limb;
-  w.CL = p; p += 2 * limb;
   w.Y = p; p += 2 * E.k * limb;
   w.R0 = p;
   return w;
@@ -88,27 +86,18 @@ static void copy_limbs(Ctx& C, uint64_t* dst, const uint64_t* src, long words) {
 
 // Forward transform of the corrections Y (npolys polys of stride k limbs,
 // limbs 0..nlimbs-1) with the key-switch combine as its epilogue.
-static void combine_into(Ctx& C, uint64_t* Y, int npolys, int nlimbs, const uint64_t* base, long base_stride,
-                         int base_polys, const uint64_t* KS, long ks_stride, int rescale_level, uint64_t* out,
-                         long out_stride, const OutPtrs* outp, cudaStream_t st = nullptr) {
-  const Engine& E = *C.E;
+static void combine_into(const Engine& E, uint64_t* Y, int npolys, int nlimbs, const uint64_t* base, long base_stride,
+                         const uint64_t* KS, long ks_stride, int rescale_level, const OutPtrs& outp, cudaStream_t st) {
   NttIo io;
   io.epi.mode = kEpiCombine;
   io.epi.base = base;
   io.epi.base_stride = base_stride;
-  io.epi.base_polys = base ? base_polys : 0;
   io.epi.ks = KS;
   io.epi.ks_stride = ks_stride;
   io.epi.binv = E.rns.moddown_binv;
   io.epi.resc = rescale_level > 0 ? E.rns.resc_inv + (long)rescale_level * E.k : nullptr;
-  if (outp) {
-    io.epi.use_ptrs = 1;
-    io.epi.outp = *outp;
-  } else {
-    io.epi.out = out;
-    io.epi.out_stride = out_stride;
-  }
-  ntt_batch_io(E, Y, npolys, 0, nlimbs, E.k, true, io, st ? st : C.stream);
+  io.epi.outp = outp;
+  ntt_batch_io(E, Y, npolys, 0, nlimbs, E.k, true, io, st);
 }
 
 // Key switch of a DGT context's automorphisms, on the Q limbs 0..level of x,
@@ -400,7 +389,7 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
     xform(E, tk, U, 2 * n, level, 1, 1, false, st);
     rescale_corrections(E, KS + (long)m * N, ks, U, N, CL, N, Y, half, 2 * n, level, st, unscaled);
     if (fuse & kFuseCombine) {
-      combine_into(C, Y, 2 * n, level, D, half, 2 * n, KS, ks, level, nullptr, 0, &outp, st);
+      combine_into(E, Y, 2 * n, level, D, half, KS, ks, level, outp, st);
     } else {
       xform(E, tk, Y, 2 * n, 0, level, k, true, st);
       ks_combine_ptr(E, outp, D, half, KS, ks, Y, half, level, 2 * n, level, st);
@@ -408,7 +397,7 @@ static void hmult_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* con
   } else {
     moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st, unscaled);
     if (fuse & kFuseCombine) {
-      combine_into(C, Y, 2 * n, m, D, half, 2 * n, KS, ks, 0, nullptr, 0, &outp, st);
+      combine_into(E, Y, 2 * n, m, D, half, KS, ks, 0, outp, st);
     } else {
       xform(E, tk, Y, 2 * n, 0, m, k, true, st);
       ks_combine_ptr(E, outp, D, half, KS, ks, Y, half, m, 2 * n, 0, st);
@@ -610,7 +599,7 @@ static void galois_group(Ctx& C, cudaStream_t st, uint64_t* p, int n, aoa_ct* co
   if (one_key)                                   // each key word read once for the group
     keyswitch_mul_batch_op(E, nullptr, 0, UB, (long)kl * N, keys[0]->d, KS + (long)m * N, ks, n, 0, st);
   else
-    keyswitch_mul_keys_op(E, nullptr, 0, UB, (long)kl * N, kp, KS + (long)m * N, ks, n, 0, st);
+    keyswitch_mul_keys_op(E, UB, (long)kl * N, kp, KS + (long)m * N, ks, n, st);
   io.src = nullptr;
   ntt_batch_io(E, KS + (long)m * N, 2 * n, k, kl, k + kl, false, io, st);
   moddown_conv(E, KS + (long)m * N, ks, Y, half, 2 * n, m, st, true);

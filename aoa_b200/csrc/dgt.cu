@@ -165,14 +165,6 @@ __device__ __forceinline__ void gi_tensor_at(const uint64_t* a, long a_half, con
   d1[off + H] = sub_mod(si, add_mod(e0i, e2i, q), q);
 }
 
-__global__ void gi_tensor(const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0, uint64_t* d1,
-                          uint64_t* d2, int H, const PrimeConst* __restrict__ pc) {
-  pdl_begin();
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= H) return;
-  gi_tensor_at(a, a_half, b, b_half, d0, d1, d2, H, pc, n, blockIdx.y);
-}
-
 // the tensor of op z = blockIdx.z of a batch: operands ptr.a[z] / ptr.b[z]
 // ([c0 | c1], stride half), outputs D0 = D, D1 = D + n half, D2 = D + 2n half
 // at op stride half
@@ -392,12 +384,6 @@ void gi_mul_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as
                int prime0, int nlimbs, int npolys, cudaStream_t st) {
   if (nlimbs <= 0 || npolys <= 0) return;
   launch_pdl(gi_mul, gi_grid(E, nlimbs * npolys), 256, 0, st, c, cs, a, as, b, bs, prime0, npolys, (int)(E.N / 2), E.d_pc);
-  AOA_CHECK_LAUNCH();
-}
-
-void gi_tensor_op(const Engine& E, const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0,
-                  uint64_t* d1, uint64_t* d2, int nlimbs, cudaStream_t st) {
-  launch_pdl(gi_tensor, gi_grid(E, nlimbs), 256, 0, st, a, a_half, b, b_half, d0, d1, d2, (int)(E.N / 2), E.d_pc);
   AOA_CHECK_LAUNCH();
 }
 

@@ -22,7 +22,7 @@
 // registers, exchanges once through (swizzled) shared memory and does the
 // low-digit stages in registers.  Global loads and stores are coalesced in both
 // passes.  Passes run in place; the host launches them over chunks of whole
-// polys of at most the engine's chunk size (default 1 GiB: the passes are bound
+// polys of at most the engine's chunk size (default 4 GiB: the passes are bound
 // by integer arithmetic, so fewer launch tails pay more than keeping the
 // column-pass output in L2 for the row pass).
 #pragma once
@@ -363,12 +363,11 @@ __device__ __forceinline__ void epi_store(const NttEpi& e, long N, long p, int l
   } else {
     const uint64_t q = P.q;
     const uint64_t kv = e.ks[p * e.ks_stride + off];
-    const uint64_t bv = p < e.base_polys ? e.base[p * e.base_stride + off] : 0;
+    const uint64_t bv = e.base[p * e.base_stride + off];
     uint64_t r;
     if (e.resc) r = shoup(sub_mod(add_mod(bv, shoup(kv, e.binv[prime], q), q), v, q), e.resc[prime], q);
     else r = add_mod(bv, shoup(sub_mod(kv, v, q), e.binv[prime], q), q);
-    uint64_t* o = e.use_ptrs ? e.outp.p[p] : e.out + p * e.out_stride;
-    o[off] = r;
+    e.outp.p[p][off] = r;
   }
 }
 
@@ -969,7 +968,7 @@ static void launch_rows(const Engine& E, const NttBatch& b, bool fwd, cudaStream
 #define AOA_NTT_SIZES(X) X(5) X(6) X(7) X(8) X(9) X(10)
 
 // Tile width choice (DIV) for a launch: the engine's tuning for lazy
-// transforms; strict transforms (primes of 62 bits or more) use the widest.
+// transforms; canonical ones (primes of 2^60 and more) use the widest.
 template <int LAZY>
 static int tile_div(int knob) { return LAZY ? std::max(0, std::min(2, knob)) : 0; }
 

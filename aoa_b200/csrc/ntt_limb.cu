@@ -124,7 +124,7 @@ __device__ __forceinline__ void sts64_cluster(uint32_t a, uint64_t v) {
   asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
 
-__device__ __forceinline__ long galois_source(long p, long g, int log_n) {   // automorph_ntt's permutation
+__device__ __forceinline__ long galois_source(long p, long g, int log_n) {   // automorph_ntt_batch's permutation
   const uint32_t br = __brev((uint32_t)p) >> (32 - log_n);
   const long e = ((2L * br + 1) * g) & ((2L << log_n) - 1);
   return (long)(__brev((uint32_t)((e - 1) >> 1)) >> (32 - log_n));

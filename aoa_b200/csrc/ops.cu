@@ -45,19 +45,6 @@ __global__ void ew_binary(Limbs c, CLimbs a, CLimbs b, int op, int prime0, const
   c.p[blockIdx.z * c.poly_stride + off] = r;
 }
 
-// c = a (op) s with a per-limb scalar s[l] (already reduced mod its prime);
-// op: 0 add, 1 sub, 2 mul
-__global__ void ew_scalar(Limbs c, CLimbs a, const uint64_t* s, int op, int prime0, const PrimeConst* pc,
-                          int log_n) {
-  pdl_begin();
-  const long N = 1L << log_n;
-  const long off = (long)blockIdx.y * N + coef_index();
-  const PrimeConst& P = pc[prime0 + blockIdx.y];
-  const uint64_t x = a.p[blockIdx.z * a.poly_stride + off], y = s[blockIdx.y];
-  c.p[blockIdx.z * c.poly_stride + off] =
-      op == 0 ? add_mod(x, y, P.q) : op == 1 ? sub_mod(x, y, P.q) : mul_mod(x, y, P);
-}
-
 // d = a * b + c  (ntt_vector_seqop)
 __global__ void ew_muladd(Limbs d, CLimbs a, CLimbs b, CLimbs c, int prime0, const PrimeConst* pc, int log_n) {
   pdl_begin();
@@ -118,43 +105,6 @@ __device__ __forceinline__ void tensor_ew(const uint64_t* a, long a_half, const 
   }
 }
 
-__global__ void hmult_tensor(const uint64_t* a, const uint64_t* b, long a_half, long b_half, uint64_t* d0,
-                             uint64_t* d1, uint64_t* d2, const PrimeConst* pc, int log_n) {
-  pdl_begin();
-  const long limb = (long)blockIdx.y << log_n;
-  const PrimeConst P = pc[blockIdx.y];
-  tensor_ew(a + limb, a_half, b + limb, b_half, d0 + limb, d1 + limb, d2 + limb, P);
-}
-
-// Key-switch products over the QB limbs of the extended d2 (transform domain):
-//   k0 = x * key_b,  k1 = x * key_a
-// x limb l < nq lives at xq + l*N (prime l), limb nq + j at xb + j*N (prime K + j);
-// the key is [b | a], each (k + kl) limbs in the reference's QB layout.
-__global__ void keyswitch_mul(const uint64_t* xq, const uint64_t* xb, const uint64_t* key, long key_half,
-                              uint64_t* k0, uint64_t* k1, int nq, int K, const PrimeConst* pc, int log_n) {
-  pdl_begin();
-  const long N = 1L << log_n;
-  const int l = blockIdx.y;
-  const int prime = l < nq ? l : K + (l - nq);
-  const uint64_t* x = l < nq ? xq + (long)l * N : xb + (long)(l - nq) * N;
-  const uint64_t* kbp = key + (long)prime * N;
-  const PrimeConst P = pc[prime];
-  uint64_t xv[kEwPer], kb[kEwPer], ka[kEwPer];
-#pragma unroll
-  for (int u = 0; u < kEwPer; u++) {
-    const long c = coef_u(u);
-    xv[u] = x[c];
-    kb[u] = kbp[c];
-    ka[u] = kbp[key_half + c];
-  }
-#pragma unroll
-  for (int u = 0; u < kEwPer; u++) {
-    const long c = coef_u(u);
-    k0[(long)l * N + c] = mul_mod(xv[u], kb[u], P);
-    k1[(long)l * N + c] = mul_mod(xv[u], ka[u], P);
-  }
-}
-
 // Coefficient-domain automorphism X -> X^g (g odd, mod 2N) with the
 // negacyclic sign (execute_rotation, encoder.cu:300-322).
 __global__ void automorph_coef(uint64_t* out, const uint64_t* in, long poly_stride, long galois,
@@ -169,26 +119,13 @@ __global__ void automorph_coef(uint64_t* out, const uint64_t* in, long poly_stri
   out[off + t] = v;
 }
 
-// Transform-domain automorphism: a permutation of the evaluation points
-// psi^(2 br(p) + 1) -> psi^((2 br(p) + 1) g).  Output position p reads the
-// input position holding the evaluation at psi^((2 br(p)+1) g).
-__global__ void automorph_ntt(uint64_t* out, const uint64_t* in, long poly_stride, long galois, int log_n) {
-  pdl_begin();
-  const long N = 1L << log_n;
-  const long p = coef_index();
-  const long off = blockIdx.z * poly_stride + (long)blockIdx.y * N;
-  const uint32_t br = __brev((uint32_t)p) >> (32 - log_n);
-  const long e = ((2L * br + 1) * galois) & (2 * N - 1);   // odd exponent mod 2N
-  const long src_br = (e - 1) >> 1;
-  const long src = __brev((uint32_t)src_br) >> (32 - log_n);
-  out[off + p] = in[off + src];
-}
-
 // ---- batched variants (one launch for a batch of ciphertexts) ---------------------
 
-// NTT-domain automorphism of both polys of ciphertext z = blockIdx.z / 2
-// (poly blockIdx.z % 2, stride half) into out: poly 0 of every op first
-// (op stride half), then poly 1 (block offset n*half).
+// Transform-domain automorphism: a permutation of the evaluation points
+// psi^(2 br(p) + 1) -> psi^((2 br(p) + 1) g); output position p reads the input
+// position holding the evaluation at psi^((2 br(p) + 1) g).  Both polys of
+// ciphertext z = blockIdx.z / 2 (poly blockIdx.z % 2, stride half) into out: poly 0
+// of every op first (op stride half), then poly 1 (block offset n*half).
 __global__ void automorph_ntt_batch(CtPtrs ptr, long half, uint64_t* out, int n, GaloisList gl, int log_n) {
   pdl_begin();
   const long N = 1L << log_n;
@@ -213,9 +150,11 @@ __global__ void hmult_tensor_batch(CtPtrs ptr, long half, uint64_t* D, int n, co
   tensor_ew(ptr.a[z] + limb, half, ptr.b[z] + limb, half, d, d + nh, d + 2 * nh, P);
 }
 
-// key products for op z: x limbs (Q part at xq + z*xq_stride, B part at
-// xb + z*xb_stride) times the key; k0 of op z at k + z*k_stride, k1 at
-// k + (n + z)*k_stride.
+// Key-switch products over the QB limbs of the extended d2 (transform domain),
+// k0 = x * key_b, k1 = x * key_a, for op z: limb l < nq of x at xq + z*xq_stride +
+// l*N (prime l), limb nq + j at xb + z*xb_stride + j*N (prime K + j); the key is
+// [b | a], each (k + kl) limbs in the reference's QB layout; k0 at k + z*k_stride,
+// k1 at k + (n + z)*k_stride.
 // One thread per (limb, kEwPer coefficients) loops over the n ops, so that
 // each key word is read from memory once per launch.
 __global__ void keyswitch_mul_batch(const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
@@ -250,17 +189,16 @@ __global__ void keyswitch_mul_batch(const uint64_t* xq, long xq_stride, const ui
   }
 }
 
-// key products with a key per op: op z's x limbs times keys.k[z] (the same
-// layout as keyswitch_mul_batch; each op's key words are read for that op)
-__global__ void keyswitch_mul_keys(const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
-                                   KeyPtrs keys, long key_half, uint64_t* k, long k_stride, int n, int nq, int K,
-                                   const PrimeConst* pc, int log_n) {
+// the special limbs' key products with a key per op: op z's limbs at xb +
+// z*xb_stride times keys.k[z] (outputs as in keyswitch_mul_batch; each op's key
+// words are read for that op)
+__global__ void keyswitch_mul_keys(const uint64_t* xb, long xb_stride, KeyPtrs keys, long key_half, uint64_t* k,
+                                   long k_stride, int n, int K, const PrimeConst* pc, int log_n) {
   pdl_begin();
   const long N = 1L << log_n;
   const int l = blockIdx.y;
-  const int prime = l < nq ? l : K + (l - nq);
-  const uint64_t* x = l < nq ? xq + (long)l * N : xb + (long)(l - nq) * N;
-  const long xs = l < nq ? xq_stride : xb_stride;
+  const int prime = K + l;
+  const uint64_t* x = xb + (long)l * N;
   const PrimeConst P = pc[prime];
   uint64_t* o = k + (long)l * N;
   for (int z = 0; z < n; z++) {
@@ -269,7 +207,7 @@ __global__ void keyswitch_mul_keys(const uint64_t* xq, long xq_stride, const uin
 #pragma unroll
     for (int u = 0; u < kEwPer; u++) {
       const long c = coef_u(u);
-      v[u] = x[z * xs + c];
+      v[u] = x[z * xb_stride + c];
       kb[u] = kbp[c];
       ka[u] = kbp[key_half + c];
     }
@@ -295,25 +233,11 @@ void ew_binary_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long
   AOA_CHECK_LAUNCH();
 }
 
-void ew_scalar_op(const Engine& E, uint64_t* c, long cs, const uint64_t* a, long as, const uint64_t* d_scalars,
-                  int op, int prime0, int nlimbs, int npolys, cudaStream_t st) {
-  if (nlimbs <= 0 || npolys <= 0) return;
-  launch_pdl(ew_scalar, ew_grid(E, nlimbs, npolys), 256, 0, st, Limbs{c, cs}, CLimbs{a, as}, d_scalars, op, prime0,
-                                                        E.d_pc, E.log_n);
-  AOA_CHECK_LAUNCH();
-}
-
 void ew_muladd_op(const Engine& E, uint64_t* d, long ds, const uint64_t* a, long as, const uint64_t* b, long bs,
                   const uint64_t* c, long cs, int prime0, int nlimbs, int npolys, cudaStream_t st) {
   if (nlimbs <= 0 || npolys <= 0) return;
   launch_pdl(ew_muladd, ew_grid(E, nlimbs, npolys), 256, 0, st, Limbs{d, ds}, CLimbs{a, as}, CLimbs{b, bs},
                                                         CLimbs{c, cs}, prime0, E.d_pc, E.log_n);
-  AOA_CHECK_LAUNCH();
-}
-
-void tensor_op(const Engine& E, const uint64_t* a, long a_half, const uint64_t* b, long b_half, uint64_t* d0,
-               uint64_t* d1, uint64_t* d2, int nlimbs, cudaStream_t st) {
-  launch_pdl(hmult_tensor, ew4_grid(E, nlimbs, 1), 256, 0, st, a, b, a_half, b_half, d0, d1, d2, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
@@ -331,14 +255,6 @@ void keyswitch_mul_batch_op(const Engine& E, const uint64_t* xq, long xq_stride,
   AOA_CHECK_LAUNCH();
 }
 
-void keyswitch_mul_op(const Engine& E, const uint64_t* xq, const uint64_t* xb, const uint64_t* key, uint64_t* k0,
-                      uint64_t* k1, int nq, cudaStream_t st, int nb) {
-  const long half = (long)E.nprimes * E.N;
-  if (nb < 0) nb = E.kl;
-  launch_pdl(keyswitch_mul, ew4_grid(E, nq + nb, 1), 256, 0, st, xq, xb, key, half, k0, k1, nq, E.k, E.d_pc, E.log_n);
-  AOA_CHECK_LAUNCH();
-}
-
 void automorph_coef_op(const Engine& E, uint64_t* out, const uint64_t* in, long poly_stride, long galois,
                        int nlimbs, int npolys, cudaStream_t st) {
   launch_pdl(automorph_coef, ew_grid(E, nlimbs, npolys), 256, 0, st, out, in, poly_stride, galois, E.d_pc, E.log_n);
@@ -351,17 +267,10 @@ void automorph_ntt_batch_op(const Engine& E, const CtPtrs& ptr, long half, uint6
   AOA_CHECK_LAUNCH();
 }
 
-void keyswitch_mul_keys_op(const Engine& E, const uint64_t* xq, long xq_stride, const uint64_t* xb, long xb_stride,
-                           const KeyPtrs& keys, uint64_t* k, long k_stride, int n, int nq, cudaStream_t st) {
-  const long half = (long)E.nprimes * E.N;
-  launch_pdl(keyswitch_mul_keys, ew4_grid(E, nq + E.kl, 1), 256, 0, st, xq, xq_stride, xb, xb_stride, keys, half, k, k_stride,
-                                                                 n, nq, E.k, E.d_pc, E.log_n);
-  AOA_CHECK_LAUNCH();
-}
-
-void automorph_ntt_op(const Engine& E, uint64_t* out, const uint64_t* in, long poly_stride, long galois,
-                      int nlimbs, int npolys, cudaStream_t st) {
-  launch_pdl(automorph_ntt, ew_grid(E, nlimbs, npolys), 256, 0, st, out, in, poly_stride, galois, E.log_n);
+void keyswitch_mul_keys_op(const Engine& E, const uint64_t* xb, long xb_stride, const KeyPtrs& keys, uint64_t* k,
+                           long k_stride, int n, cudaStream_t st) {
+  launch_pdl(keyswitch_mul_keys, ew4_grid(E, E.kl, 1), 256, 0, st, xb, xb_stride, keys, (long)E.nprimes * E.N, k,
+             k_stride, n, E.k, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 

@@ -680,7 +680,7 @@ __global__ void ks_combine_kernel(uint64_t* out, long out_stride, const uint64_t
 }
 
 // Same epilogue writing poly p to outp.p[p] (a list of output polys).
-__global__ void ks_combine_ptr_kernel(OutPtrs outp, const uint64_t* base, long base_stride, int base_polys,
+__global__ void ks_combine_ptr_kernel(OutPtrs outp, const uint64_t* base, long base_stride,
                                       const uint64_t* k, long k_stride, const uint64_t* y, long y_stride,
                                       const ShoupW* binv, const ShoupW* resc, const PrimeConst* pc, int log_n) {
   pdl_begin();
@@ -691,7 +691,7 @@ __global__ void ks_combine_ptr_kernel(OutPtrs outp, const uint64_t* base, long b
   const ShoupW bi = binv[i], rs = resc ? resc[i] : ShoupW{0, 0};
   const uint64_t* kp = k + p * k_stride + limb;
   const uint64_t* yp = y + p * y_stride + limb;
-  const uint64_t* bp = base && p < base_polys ? base + p * base_stride + limb : nullptr;
+  const uint64_t* bp = base + p * base_stride + limb;
   uint64_t* op = outp.p[p] + limb;
   uint64_t kv[kCombPer], yv[kCombPer], bv[kCombPer];
 #pragma unroll
@@ -699,7 +699,7 @@ __global__ void ks_combine_ptr_kernel(OutPtrs outp, const uint64_t* base, long b
     const long c = ((long)blockIdx.x * kCombPer + u) * blockDim.x + threadIdx.x;
     kv[u] = kp[c];
     yv[u] = yp[c];
-    bv[u] = bp ? bp[c] : 0;
+    bv[u] = bp[c];
   }
 #pragma unroll
   for (int u = 0; u < kCombPer; u++) {
@@ -710,12 +710,12 @@ __global__ void ks_combine_ptr_kernel(OutPtrs outp, const uint64_t* base, long b
 
 void ks_combine_ptr(const Engine& E, const OutPtrs& outp, const uint64_t* base, long base_stride, const uint64_t* k,
                     long k_stride, const uint64_t* y, long y_stride, int nlimbs, int npolys, int rescale_level,
-                    cudaStream_t st, int base_polys) {
+                    cudaStream_t st) {
   if (nlimbs <= 0) return;
   dim3 grid(E.N / (256 * kCombPer), nlimbs, npolys);
   const ShoupW* resc = rescale_level > 0 ? E.rns.resc_inv + (long)rescale_level * E.k : nullptr;
-  launch_pdl(ks_combine_ptr_kernel, grid, 256, 0, st, outp, base, base_stride, base_polys < 0 ? npolys : base_polys, k,
-                                              k_stride, y, y_stride, E.rns.moddown_binv, resc, E.d_pc, E.log_n);
+  launch_pdl(ks_combine_ptr_kernel, grid, 256, 0, st, outp, base, base_stride, k, k_stride, y,
+             y_stride, E.rns.moddown_binv, resc, E.d_pc, E.log_n);
   AOA_CHECK_LAUNCH();
 }
 
