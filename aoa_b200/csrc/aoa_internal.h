@@ -211,8 +211,10 @@ void note_launch();
 // calls are chains of kernels of a few microseconds, bound by the gap between
 // them: HMult at 2^12 (16 launches) 88.1 -> 50.1 us, at 2^16 (30 limbs) 373.8 ->
 // 355.0 us, a rotation at 2^13 92.0 -> 55.6 us.
+// early: false launches it the ordinary way (pdl_begin() then lets the next one be
+// set up, no more).
 template <class... P, class... A>
-void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+void launch_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -222,9 +224,13 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaSt
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   AOA_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
   note_launch();
+}
+template <class... P, class... A>
+void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  launch_early(true, kernel, grid, block, smem, st, args...);
 }
 
 // C-ABI error plumbing (engine.cu)

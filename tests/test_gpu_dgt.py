@@ -83,6 +83,23 @@ def test_dgt_split_knob_keeps_results(dgt_table, log_n):
     E.tune("dgt_split", 1)
 
 
+@pytest.mark.parametrize("log_n,npolys", [(13, 102), (13, 103), (16, 13)])
+def test_dgt_of_large_calls(dgt_table, log_n, npolys):
+    """On both sides of the twist's launch rule (16384 CTAs: 16 a limb at 2^13, 128 at 2^16; 10 limbs a poly)."""
+    require_gpu()
+    aoa, E, ctx, D, _ = _setup(dgt_table, log_n, 5, 5, 48)
+    rng = np.random.default_rng(npolys)
+    x = uniform_residues(rng, E.primes, E.N)
+    xs = np.stack([np.roll(x, p, axis=1) % np.array(E.primes, dtype=np.uint64)[:, None] for p in range(npolys)])
+    d = ctx.upload(xs)
+    ctx.dgt_fwd(d, npolys, 0, 10)
+    got = d.numpy()
+    for p in (0, npolys - 1):
+        assert np.array_equal(got[p], unfold(D.fwd(fold(xs[p]))))
+    ctx.dgt_inv(d, npolys, 0, 10)
+    assert np.array_equal(d.numpy(), xs)
+
+
 def test_gi_layout_and_mul(dgt_table):
     require_gpu()
     aoa, E, ctx, D, _ = _setup(dgt_table, 12, 2, 2, 55)
