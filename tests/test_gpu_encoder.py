@@ -152,3 +152,23 @@ def test_encoder_rejects_bad_arguments():
     d = ctx.alloc((E.k, E.N))
     with pytest.raises(aoa.AoaError):
         aoa.ckks_decode(ctx, d, 6, 1 << 40)
+
+
+def test_encode_and_rescale_of_many_limbs():
+    """On both sides of the launch rules at 2^16 (256 CTAs a limb): 32 and 33 encoded limbs, a rescale of 32 and 33."""
+    require_gpu()
+    aoa, E, ctx, o = _setup(16, nq=34, nb=1)
+    rng = np.random.default_rng(3)
+    vals = _values(rng, 8)
+    want = o.encode(vals, 1 << 40)
+    for nlimbs in (32, 33):
+        got, _ = aoa.ckks_encode(ctx, vals, scale=1 << 40, nlimbs=nlimbs)
+        assert np.array_equal(got.numpy(), want[:nlimbs])
+    c0, c1 = uniform_residues(rng, o.primes[:34], o.N), uniform_residues(rng, o.primes[:34], o.N)
+    for level in (32, 33):
+        ct = aoa.Ciphertext.from_residues(ctx, c0, c1, slots=8, scale=1 << 60, domain=aoa.AOA_COEF)
+        ct.set(level, 8, 1 << 60, aoa.AOA_COEF)
+        aoa.ckks_rescale(ctx, ct)
+        w0, w1 = o.rescale(c0, c1, level)
+        g0, g1 = ct.download(nlimbs=level, domain=aoa.AOA_COEF)
+        assert np.array_equal(g0, w0[:level]) and np.array_equal(g1, w1[:level])
