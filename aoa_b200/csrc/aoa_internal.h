@@ -302,6 +302,7 @@ struct NttIo {
   long src_poly_stride = 0;
   bool unscaled = false;
   int prime_gap = 0;       // limbs after the first are under primes this much further on
+  bool part = false;       // one run of a call whose primes are of several kinds (ntt_batch_tables)
   NttEpi epi;
 };
 void ntt_init(Engine& E);

@@ -136,6 +136,7 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
       if (io) run = *io;
       if (run.src) run.src += (long)l0 * n;
       run.epi.limb_base += l0;
+      run.part = true;
       if (l0) run.prime_gap = 0;                 // it is in the run's first prime
       ntt_batch_tables(E, T2, data + (long)l0 * n, npolys, first_prime + (l0 >> T.prime_shift) + (l0 ? gap : 0),
                        l1 - l0, poly_stride, forward, st, &run);
@@ -157,6 +158,7 @@ void ntt_batch_tables(const Engine& E, const NttTables& T, uint64_t* data, int n
   b.first_prime = first_prime; b.prime_shift = T.prime_shift; b.poly_stride = poly_stride;
   b.src = nullptr; b.src_poly_stride = 0; b.poly_base = 0; b.use_tma = 0;
   b.unscaled = io && io->unscaled;
+  b.alone = !(io && io->part);
   b.prime_gap = gap;
   const long n = 1L << T.log_n;
   if ((b.unscaled && forward) || ((b.unscaled || gap) && T.log_n < 10))

@@ -397,6 +397,7 @@ struct NttBatch {
   int poly_base;           // poly index of the launch's first poly within the call
   int spin;                // polls of a bounded wait for this kernel's own copies (engine knob)
   bool unscaled;           // inverse column pass: without N^-1
+  bool alone;              // the launches are a whole call's, not one kind's run of it (host only)
   int use_tma;             // column pass: tiles by one tensor-map load (the kernel's tmap argument)
   __device__ __forceinline__ int prime_of(int limb) const {
     return first_prime + (limb >> prime_shift) + (limb ? prime_gap : 0);
@@ -962,7 +963,18 @@ static void launch_rows(const Engine& E, const NttBatch& b, bool fwd, cudaStream
   if (R % Tl::ROWS) throw AoaError(AOA_ERR_BAD_PARAM, "ntt: row tile does not divide R");
   dim3 grid(R / Tl::ROWS, ctas_per_tile(E, rows_apart(b.npolys), R / Tl::ROWS, b.nitems, Tl::MIN_BLOCKS));
   if (fwd) launch_pdl(ntt_rows<LOG_C, DIV, LAZY, true>, grid, Tl::THREADS, Tl::SMEM, st, b, epi);
-  else launch_pdl(ntt_rows<LOG_C, DIV, LAZY, false>, grid, Tl::THREADS, Tl::SMEM, st, b, epi);
+  else {
+    // Launched early, the CTAs of a call's first pass fill the SMs on which the kernel
+    // before ends first.  Between one CTA per SM and half of the chip's places that
+    // leaves other SMs idle, with rows of 512 points and more for longer than the gap
+    // it closes (inverse DGT of 2^17, 55-bit primes, us, early -> not: 2 limbs, 128
+    // CTAs, 20.9 -> 20.6; 4 limbs 34.3 -> 25.7; 6 limbs, 384, 40.0 -> 32.8; 8 limbs,
+    // 512, 37.9 -> 39.0; 62-bit primes 2 limbs, 64 CTAs, 31.6 -> 34.9; 4 limbs 43.9 ->
+    // 35.4).
+    const long ctas = (long)grid.x * grid.y;
+    const bool early = LOG_C < 9 || !b.alone || ctas < 100 || 2 * ctas > (long)E.num_sms * Tl::MIN_BLOCKS;
+    launch_early(early, ntt_rows<LOG_C, DIV, LAZY, false>, grid, Tl::THREADS, Tl::SMEM, st, b, epi);
+  }
 }
 
 #define AOA_NTT_SIZES(X) X(5) X(6) X(7) X(8) X(9) X(10)

@@ -360,3 +360,23 @@ def test_dgt_hmult_batch_matches_oracle_and_per_call(dgt_table, rescale):
         s0, s1 = single.download(nlimbs=nl, domain=aoa.AOA_DGT)
         b0, b1 = outs[z].download(nlimbs=nl, domain=aoa.AOA_DGT)
         assert np.array_equal(s0, b0) and np.array_equal(s1, b1), z
+
+
+def test_inverse_of_few_limbs_of_the_largest_ring():
+    """Each limb count's launches give the words of one large call (forward, then inverse back)."""
+    require_gpu()
+    import aoa_b200 as aoa
+    from aoa_b200 import params
+    ps = params.ntt_primes(63, 1 << 18, 1) + params.ntt_primes(55, 1 << 18, 11)
+    E = aoa.Engine(17, ps, [])
+    ctx = aoa.Context(E)
+    x = uniform_residues(np.random.default_rng(5), ps, E.N)
+    d = ctx.upload(x)
+    ctx.dgt_fwd(d, 1, 0, 12)
+    X = d.numpy()
+    ctx.dgt_inv(d, 1, 0, 12)
+    assert np.array_equal(d.numpy(), x)
+    for first, n in ((0, 1), (0, 2), (1, 1), (1, 2), (1, 4), (1, 6), (1, 8), (1, 11)):
+        d = ctx.upload(X[first:first + n])
+        ctx.dgt_inv(d, 1, first, n)
+        assert np.array_equal(d.numpy(), x[first:first + n]), (first, n)
