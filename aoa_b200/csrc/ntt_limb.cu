@@ -567,9 +567,11 @@ void limb_init(const Engine&) {
 // passes, which have the higher throughput once the chip is full.  Measured on
 // both sides of each line (us, two passes -> whole limbs, one B200):
 //   forward, one lazy kind: 2^11, 1024 limbs 40 -> 31; 2^12, 112 11.1 -> 10.1, 150
-//     12.2 -> 13.3, 336 20.7 -> 23.8; 2^13, 64 13.9 -> 12.3, 80 16.2 -> 16.5, 128
-//     18.4 -> 21.6; 2^14, 32 (a cluster of four on every SM) 12.5 -> 11.0, 36 12.6
-//     -> 21.0, 64 21.4 -> 22.1; 2^15, 1 to 8 8.5 -> 11.0;
+//     12.2 -> 13.3, 336 20.7 -> 23.8; 2^13, 64 13.9 -> 12.3, 96 16.4 -> 16.6 (four
+//     HMults with 68 limbs 93.0 -> 91.4), 128 18.4 -> 21.6; 2^14, 32 (a cluster of
+//     four on every SM) 12.5 -> 11.0, 36 12.6 -> 21.0, 64 21.4 -> 22.1; 2^15, 1 to 8
+//     8.5 -> 11.0, but within an HMult of 4 or 5 limbs, whose corrections are 6 or 8,
+//     114.4 -> 111.9 and 123.5 -> 118.4;
 //   DGT limbs of one lazy kind, with the twist: 2^11, 512 22.3 -> 21.6, 608 24.0 ->
 //     26.3; 2^12, 448 forward 37.2 -> 38.7, inverse 41.3 -> 36.2; 2^13, 128 28.3 ->
 //     26.3, 160 31.7 -> 34.1; 2^14, 32 16.1 -> 14.4, 48 18.0 -> 26.2; 2^15, 8 17.4
@@ -585,7 +587,7 @@ void limb_init(const Engine&) {
 //     -> 94, 100 142 -> 152; rotation 2^14, 56 110 -> 109, 80 136 -> 140; 2^15, 16
 //     83.9 -> 85.8, 24 98 -> 110; HMult 2^15, 20 95 -> 90, 30 107 -> 98.
 bool limb_serves(const Engine& E, int log_n, long items, LimbUse use) {
-  constexpr long kMost[4][6] = {{1024, 1024, 128, 64, 32, 0},     // kLimbForward; log_n = 10 .. 15
+  constexpr long kMost[4][6] = {{1024, 1024, 128, 96, 32, 8},     // kLimbForward; log_n = 10 .. 15
                                 {1024, 512, 448, 128, 32, 8},     // kLimbCyclic
                                 {1024, 1024, 448, 128, 64, 8},    // kLimbOther
                                 {1024, 1024, 320, 112, 56, 20}};  // kLimbFused
