@@ -895,10 +895,10 @@ ntt_rows(NttBatch b, const __grid_constant__ NttEpi epi) {
 
 // large launches balance better with more, shorter-lived CTAs (the hardware
 // hands later waves to the SMs that finish first); small ones pay per CTA
-static inline int ctas_per_tile(const Engine& E, double apart, int tiles, int items, int blocks_per_sm) {
+static inline int ctas_per_tile(const Engine& E, int share, int tiles, int items, int blocks_per_sm) {
   const bool large = items >= kLargeItems;
   return ctas_per_tile(large ? E.tune.ntt_waves_large : E.tune.ntt_waves,
-                       large ? Tune{}.ntt_waves_large : Tune{}.ntt_waves, apart, E.num_sms * blocks_per_sm, tiles,
+                       large ? Tune{}.ntt_waves_large : Tune{}.ntt_waves, share, E.num_sms * blocks_per_sm, tiles,
                        items);
 }
 
@@ -940,7 +940,7 @@ static void launch_cols(const Engine& E, const NttBatch& b0, bool fwd, cudaStrea
   CUtensorMap map{};
   // a tensor-map tile load needs the rows of the tile in order (no row swizzle: W = 16)
   b.use_tma = E.tune.ntt_cols_tma && Tl::W == 16 && col_tensor_map(b, Tl::W, &map) ? 1 : 0;
-  dim3 grid(C / Tl::W, ctas_per_tile(E, cols_apart(), C / Tl::W, b.nitems, Tl::MIN_BLOCKS));
+  dim3 grid(C / Tl::W, ctas_per_tile(E, 1, C / Tl::W, b.nitems, Tl::MIN_BLOCKS));
   if (fwd) launch_pdl(ntt_cols<LOG_R, DIV, LAZY, true>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
   else if (b.unscaled) launch_pdl(ntt_cols<LOG_R, DIV, LAZY, false, true>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
   else launch_pdl(ntt_cols<LOG_R, DIV, LAZY, false>, grid, Tl::THREADS, Tl::SMEM, st, b, map);
@@ -951,7 +951,7 @@ static void launch_cols_wo(const Engine& E, const NttBatch& b, bool fwd, cudaStr
   using Tl = WoTile<LOG_R, NW>;
   const int C = 1 << b.log_c;
   if (C % Tl::W) throw AoaError(AOA_ERR_BAD_PARAM, "ntt: column tile does not divide C");
-  dim3 grid(C / Tl::W, ctas_per_tile(E, cols_apart(), C / Tl::W, b.nitems, Tl::MIN_BLOCKS));
+  dim3 grid(C / Tl::W, ctas_per_tile(E, 1, C / Tl::W, b.nitems, Tl::MIN_BLOCKS));
   if (fwd) launch_pdl(ntt_cols_wo<LOG_R, NW, true>, grid, Tl::THREADS, Tl::SMEM, st, b);
   else launch_pdl(ntt_cols_wo<LOG_R, NW, false>, grid, Tl::THREADS, Tl::SMEM, st, b);
 }
@@ -961,7 +961,7 @@ static void launch_rows(const Engine& E, const NttBatch& b, bool fwd, cudaStream
   using Tl = RowTile<LOG_C, DIV>;
   const int R = 1 << b.log_r;
   if (R % Tl::ROWS) throw AoaError(AOA_ERR_BAD_PARAM, "ntt: row tile does not divide R");
-  dim3 grid(R / Tl::ROWS, ctas_per_tile(E, rows_apart(b.npolys), R / Tl::ROWS, b.nitems, Tl::MIN_BLOCKS));
+  dim3 grid(R / Tl::ROWS, ctas_per_tile(E, b.npolys, R / Tl::ROWS, b.nitems, Tl::MIN_BLOCKS));
   if (fwd) launch_pdl(ntt_rows<LOG_C, DIV, LAZY, true>, grid, Tl::THREADS, Tl::SMEM, st, b, epi);
   else {
     // Launched early, the CTAs of a call's first pass fill the SMs on which the kernel

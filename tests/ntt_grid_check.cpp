@@ -11,12 +11,13 @@ int main() {
       for (int items = 1; items <= 3000; items += 1 + items / 8)
         for (double waves : {0.01, 0.5, 1.0, 2.0, 2.5, 8.0, 64.0})
           for (double def : {1.0, 8.0}) {
-            const double apart = items % 2 ? aoa::cols_apart() : aoa::rows_apart(1 + items % 3);
-            const int g = aoa::ctas_per_tile(waves, def, apart, resident, tiles, items);
+            const int share = 1 + items % 5;
+            const int g = aoa::ctas_per_tile(waves, def, share, resident, tiles, items);
             const double want = waves * resident / tiles;   // CTAs per tile column of that many waves
-            bool ok = g >= 1 && g <= items;
-            if (waves == def && items * (double)tiles <= apart * resident) ok = ok && g == items;
-            else ok = ok && (g == 1 || g <= want) && (g == items || g + 1 > want);
+            const double mean = (double)items * tiles / resident;
+            const bool each = g == items, wave = (g == 1 || g <= want) && (each || g + 1 > want);
+            bool ok = g >= 1 && g <= items && (wave || (each && waves == def && mean <= 2.5));
+            if (waves == def && (share == 1 ? mean <= 2.5 : share > 3 && mean <= 1.2)) ok = ok && each;
             if (!ok) {
               std::printf("waves %g (default %g), resident %d, tiles %d, items %d: %d\n", waves, def, resident, tiles,
                           items, g);
